@@ -236,6 +236,93 @@ __global__ void orbit_positions_kernel(const OrbitDev o, float* pos, double* pos
   }
 }
 
+// FP64 positions of circular orbits (e = 0), a block's threads on (snapshot, satellite).
+// Bound by the FP64 pipe (2 lanes per SM and clock), so each block evaluates what its
+// positions share once: sin and cos of the reference satellite's argument of latitude per
+// snapshot, and of the RAAN per orbit.  A satellite's lead angle is 2 asin(x), x = d / 2a, and
+//   cos(2 asin x) = 1 - 2 x^2,  sin(2 asin x) = 2 x sqrt(1 - x^2)
+// turn it in by two products; with e = 0 the true anomaly is the mean anomaly itself.  About
+// 27 FP64 operations a position instead of ~600: 65,536 snapshots of 8 satellites 348 -> 38 us.
+struct OrbitF64 {
+  double step, slope1[32], slope2[32];  // 2 pi / (res - 1); linspace steps of the separation ramps
+  double inv2a;                         // 1 / (2a * 1e3)
+  double ci, si;                        // inclination
+  int per_block;                        // snapshots per block
+};
+constexpr int F64_THREADS = 512;
+constexpr int F64_RAAN_TAB = 4;  // orbits per block with a precomputed RAAN
+
+__device__ __forceinline__ double raan64(const OrbitDev& o, int k) {
+  const double d2r = kPi / 180.0;
+  return (double)k * d2r * o.raan_step + (double)(o.index - 1) * (double)o.orbit_counts * d2r * o.raan_step;
+}
+
+__global__ void __launch_bounds__(F64_THREADS) orbit_positions_f64_kernel(const OrbitDev o, const OrbitF64 f, float* pos,
+                                                                          double* pos64) {
+  __shared__ double s_c[F64_THREADS / 2], s_s[F64_THREADS / 2];  // per snapshot: cos, sin of the argument of latitude
+  __shared__ int s_circle[F64_THREADS / 2];                      // its sample, -1: zero-filled
+  __shared__ double s_raan[F64_RAAN_TAB][2];
+  __shared__ int s_k0;
+  const int g0 = (int)blockIdx.x * f.per_block;
+  const int ns = min(f.per_block, o.S - g0);
+  // the table's orbits, from that of the block's first snapshot on (by the last warp, beside
+  // the snapshots' angles)
+  const int tab = (int)threadIdx.x - (F64_THREADS - 32);
+  if (tab >= 0 && tab < F64_RAAN_TAB) {
+    int c0;
+    const int k0 = window_index(o, g0, &c0) == 0 ? o.by_res.div(c0) : 0;
+    double sr, cr;
+    sincos(raan64(o, k0 + tab), &sr, &cr);
+    s_raan[tab][0] = cr;
+    s_raan[tab][1] = sr;
+    if (tab == 0) s_k0 = k0;
+  }
+  if ((int)threadIdx.x < ns) {
+    int circle;
+    const int kind = window_index(o, g0 + (int)threadIdx.x, &circle);
+    s_circle[threadIdx.x] = kind == 0 ? circle : -1;
+    if (kind == 0) {
+      const int po = circle - o.by_res.div(circle) * o.orbit_res;
+      double sn, cs;
+      sincos(f.step * (double)po + o.argp64, &sn, &cs);
+      s_c[threadIdx.x] = cs;
+      s_s[threadIdx.x] = sn;
+    }
+  }
+  __syncthreads();
+  const int ls = o.by_nsat.div((int)threadIdx.x);
+  const int sat = (int)threadIdx.x - ls * o.nsat;
+  if (ls >= ns) return;
+  const int idx = s_circle[ls];
+  double p0 = 0.0, p1 = 0.0, p2 = 0.0;
+  if (idx >= 0) {
+    const double d = idx < o.half ? fma(f.slope1[sat], (double)idx, (double)o.r1[sat])
+                                  : fma(f.slope2[sat], (double)(idx - o.half), (double)o.r2[sat]);
+    const double x = d * f.inv2a, x2 = x * x;
+    // sqrt(1 - x^2): its series to x^12 below |x| = 0.05 (the rest < 2^-57)
+    const double q =
+        x2 <= 0.0025 ? fma(-x2, fma(x2, fma(x2, fma(x2, fma(x2, fma(x2, 21.0 / 1024, 7.0 / 256), 5.0 / 128), 1.0 / 16), 1.0 / 8), 0.5), 1.0)
+                     : sqrt(1.0 - x2);
+    const double c2 = fma(-2.0, x2, 1.0), s2 = (x + x) * q;
+    const double cw = o.a64 * fma(s_c[ls], c2, -s_s[ls] * s2), sw = o.a64 * fma(s_s[ls], c2, s_c[ls] * s2);
+    const int dk = o.by_res.div(idx) - s_k0;
+    double cr, sr;
+    if (dk >= 0 && dk < F64_RAAN_TAB) {
+      cr = s_raan[dk][0];
+      sr = s_raan[dk][1];
+    } else {
+      sincos(raan64(o, s_k0 + dk), &sr, &cr);
+    }
+    const double t = sw * f.ci;
+    p0 = fma(cw, cr, -t * sr);
+    p1 = fma(cw, sr, t * cr);
+    p2 = sw * f.si;
+  }
+  const int at = 3 * (g0 * o.nsat + (int)threadIdx.x);
+  pos[at] = (float)p0; pos[at + 1] = (float)p1; pos[at + 2] = (float)p2;
+  if (pos64) { pos64[at] = p0; pos64[at + 1] = p1; pos64[at + 2] = p2; }
+}
+
 // pair q -> (m, n): ordered pairs m != n m-major (:350-353), unordered m < n.
 __device__ __forceinline__ void pair_of(int q, int nsat, int ordered, int* m, int* n) {
   if (ordered) {
@@ -287,30 +374,52 @@ __device__ __forceinline__ float baseline_coord(float diff, double lambda, float
   return ceil_quotient_exact(diff, lambda);
 }
 
-__global__ void baseline_uvw_kernel(const float* pos, const double* pos64, int64_t S, int nsat, int ordered, int npairs,
-                                    uint64_t pair_magic, double lambda, float2 scale, int rounding, float* u,
-                                    float* v, float* w, int32_t* snap, int32_t* pair) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= S * npairs) return;
-  // k / npairs by a multiply-high (magic = ceil(2^64 / npairs)), corrected once
-  int64_t g = (int64_t)__umul64hi((uint64_t)k, pair_magic);
-  int q = (int)(k - g * npairs);
-  if (q < 0) { --g; q += npairs; }
-  if (q >= npairs) { ++g; q -= npairs; }
-  int m, n;
-  pair_of(q, nsat, ordered, &m, &n);
-  float out[3];
-  for (int c = 0; c < 3; ++c) {
-    if (pos64) {
-      const double x = (pos64[(g * nsat + n) * 3 + c] - pos64[(g * nsat + m) * 3 + c]) * 1e3 / lambda;
-      out[c] = rounding ? (float)ceil(x) : (float)x;
-      continue;
-    }
-    out[c] = baseline_coord(pos[(g * nsat + n) * 3 + c] - pos[(g * nsat + m) * 3 + c], lambda, scale, rounding);
+// Baselines of a block's snapshots: their positions and the (m, n) of every pair are staged in
+// shared memory, then a thread forms every BASE_THREADS-th row.  The rows are written in order
+// (20 B each: the bound once the pair and the division are off the rows' path).  FP64
+// positions without the ceil take (p_n - p_m) * (1e3 / lambda): one FP64 product where
+// the quotient's division was ten or more (the float result differs where the two FP64 values
+// straddle a rounding boundary, a few in 10^6).  65,536 snapshots x 28 pairs: 122 -> 34 us.
+constexpr int BASE_THREADS = 256;
+constexpr int BASE_MAX_PAIRS = 32 * 31;
+
+template <class T>
+__global__ void __launch_bounds__(BASE_THREADS) baseline_uvw_kernel(const T* pos, int64_t S, int nsat, int ordered,
+                                                                   int npairs, int per_block, FastDiv by_npairs,
+                                                                   double lambda, double scale64, float2 scale,
+                                                                   int rounding, float* u, float* v, float* w,
+                                                                   int32_t* snap, int32_t* pair) {
+  extern __shared__ double s_raw[];
+  T* const s_pos = reinterpret_cast<T*>(s_raw);  // [per_block][nsat][3]
+  __shared__ int s_pair[BASE_MAX_PAIRS];
+  const int64_t g0 = (int64_t)blockIdx.x * per_block;
+  const int ns = (int)(S - g0 < per_block ? S - g0 : per_block);
+  for (int i = threadIdx.x; i < ns * nsat * 3; i += BASE_THREADS) s_pos[i] = pos[g0 * nsat * 3 + i];
+  for (int q = threadIdx.x; q < npairs; q += BASE_THREADS) {
+    int m, n;
+    pair_of(q, nsat, ordered, &m, &n);
+    s_pair[q] = m | (n << 16);
   }
-  u[k] = out[0]; v[k] = out[1]; w[k] = out[2];
-  if (snap) snap[k] = (int32_t)g;
-  if (pair) pair[k] = m | (n << 16);
+  __syncthreads();
+  for (int i = threadIdx.x; i < ns * npairs; i += BASE_THREADS) {
+    const int ls = by_npairs.div(i);
+    const int pq = s_pair[i - ls * npairs];
+    const T* const pm = s_pos + (ls * nsat + (pq & 0xffff)) * 3;
+    const T* const pn = s_pos + (ls * nsat + (pq >> 16)) * 3;
+    float out[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const T diff = pn[c] - pm[c];
+      if (sizeof(T) == sizeof(double))
+        out[c] = rounding ? (float)ceil((double)diff * 1e3 / lambda) : (float)((double)diff * scale64);
+      else
+        out[c] = baseline_coord((float)diff, lambda, scale, rounding);
+    }
+    const int64_t k = g0 * npairs + i;
+    u[k] = out[0]; v[k] = out[1]; w[k] = out[2];
+    if (snap) snap[k] = (int32_t)(g0 + ls);
+    if (pair) pair[k] = pq;
+  }
 }
 
 // ---------------------------------------------------------------- dedup
@@ -717,6 +826,22 @@ int viss_orbit_positions(const viss_orbit_cfg* cfg, float* pos, double* pos64, v
   const int64_t n = (int64_t)o.S * o.nsat;
   if (n == 0) return VISS_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (o.fp64 && o.e64 == 0.0) {
+    OrbitF64 f{};
+    f.step = 2.0 * kPi / (double)(o.orbit_res - 1);
+    for (int s = 0; s < o.nsat; ++s) {
+      f.slope1[s] = ((double)o.r2[s] - (double)o.r1[s]) / (double)(half - 1);
+      f.slope2[s] = ((double)o.r1[s] - (double)o.r2[s]) / (double)(half - 1);
+    }
+    f.inv2a = 1.0 / (2.0 * o.a64 * 1e3);
+    f.ci = cos(o.incl64);
+    f.si = sin(o.incl64);
+    f.per_block = F64_THREADS / o.nsat;
+    orbit_positions_f64_kernel<<<(unsigned)((o.S + f.per_block - 1) / f.per_block), F64_THREADS, 0, st>>>(o, f, pos,
+                                                                                                       pos64);
+    VISS_LAUNCH_CHECK("orbit_positions_f64_kernel");
+    return VISS_OK;
+  }
   orbit_positions_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(o, pos, pos64);
   VISS_LAUNCH_CHECK("orbit_positions_kernel");
   return VISS_OK;
@@ -732,9 +857,24 @@ int viss_baseline_uvw(const float* pos, const double* pos64, int64_t S, int32_t 
   const int64_t K = S * npairs;
   if (K == 0) return VISS_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const uint64_t magic = ~0ull / (uint64_t)npairs + 1;
-  baseline_uvw_kernel<<<(unsigned)((K + 255) / 256), 256, 0, st>>>(
-      pos, pos64, S, nsat, ordered, npairs, magic, lambda_m, scale_pair(lambda_m), rounding, u, v, w, snap, pair);
+  // ~2,048 rows a block (several rows a thread share its staging), and at most 24 KB of positions
+  int per_block = 2048 / npairs;
+  if (per_block > 1024 / nsat) per_block = 1024 / nsat;
+  if (per_block < 1) per_block = 1;
+  if (per_block > S) per_block = (int)S;
+  const int64_t blocks = (S + per_block - 1) / per_block;
+  if (blocks > (int64_t)INT32_MAX) return fail(VISS_ERR_RANGE, "too many snapshots");
+  FastDiv by_npairs;
+  by_npairs.set(npairs);
+  const size_t elems = (size_t)per_block * nsat * 3;
+  if (pos64)
+    baseline_uvw_kernel<double><<<(unsigned)blocks, BASE_THREADS, elems * sizeof(double), st>>>(
+        pos64, S, nsat, ordered, npairs, per_block, by_npairs, lambda_m, 1e3 / lambda_m, scale_pair(lambda_m), rounding,
+        u, v, w, snap, pair);
+  else
+    baseline_uvw_kernel<float><<<(unsigned)blocks, BASE_THREADS, elems * sizeof(float), st>>>(
+        pos, S, nsat, ordered, npairs, per_block, by_npairs, lambda_m, 1e3 / lambda_m, scale_pair(lambda_m), rounding, u,
+        v, w, snap, pair);
   VISS_LAUNCH_CHECK("baseline_uvw_kernel");
   return VISS_OK;
 }
