@@ -522,7 +522,11 @@ __global__ void dedup_hash_kernel(const float* u, const float* v, const float* w
 // and inserts a row only where its key differs from the previous snapshot's: an
 // equal key there has the smaller row index already.  Baselines move by far
 // less than a wavelength between snapshots, so most rows touch no table slot.
-constexpr int UNIQUE_RUN = 256;
+// A thread's run is at most UNIQUE_RUN snapshots, and shorter (down to UNIQUE_RUN_MIN) where
+// the pass would leave the chip's thread slots empty: the inserts are chains of dependent table
+// accesses, hidden only by other threads (403,200 snapshots of 8 satellites: 256 -> 16 a run).
+constexpr int UNIQUE_RUN = 256, UNIQUE_RUN_MIN = 16;
+constexpr int UNIQUE_CTAS = 6;  // CTAs of 256 threads per SM (40 registers)
 constexpr int UNIQUE_BATCH = 2;
 
 // Key fields of row (m, n) and row (n, m) for one coordinate: F = ceil(q) + 2^20
@@ -574,17 +578,17 @@ __device__ __forceinline__ void row_keys(const float* d, double lambda, float2 s
   *kr = ((uint64_t)fr[0] << 42) | ((uint64_t)fr[1] << 21) | (uint64_t)fr[2];
 }
 
-__global__ void __launch_bounds__(256, 6) unique_insert_kernel(const float* __restrict__ pos, int64_t S, int nsat,
-                                                            int ordered, int npairs, double lambda, float2 scale,
+__global__ void __launch_bounds__(256, UNIQUE_CTAS) unique_insert_kernel(const float* __restrict__ pos, int64_t S, int nsat,
+                                                            int ordered, int run, double lambda, float2 scale,
                                                             uint64_t* tkeys, uint32_t* tidx, uint64_t mask, int* bad,
                                                             int* overflow) {
   const int nup = nsat * (nsat - 1) / 2;  // satellite pairs m < n
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t chunk = t / nup;
   const int up = (int)(t - chunk * nup);
-  const int64_t g0 = chunk * UNIQUE_RUN;
+  const int64_t g0 = chunk * run;
   if (g0 >= S) return;
-  const int cnt = (int)(g0 + UNIQUE_RUN < S ? UNIQUE_RUN : S - g0);
+  const int cnt = (int)(g0 + run < S ? run : S - g0);
   int m, n;
   pair_of(up, nsat, 0, &m, &n);
   // row offsets within a snapshot: (m, n) and, ordered, (n, m) (pair_of's order)
@@ -642,19 +646,26 @@ constexpr int COMPACT_SLOTS = 256 * COMPACT_PER_THREAD;
 
 __global__ void __launch_bounds__(256) unique_compact_kernel(const uint64_t* tkeys, const uint32_t* tidx, int64_t T,
                                                              uint64_t* k1, uint32_t* i1,
-                                                             unsigned long long* count) {
+                                                             unsigned long long* count, int* maxdev) {
   __shared__ unsigned warp_sum[8];
   __shared__ unsigned long long block_base;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int64_t base = (int64_t)blockIdx.x * COMPACT_SLOTS + tid;
   uint64_t keys[COMPACT_PER_THREAD];
   unsigned mine = 0;
+  int dev = 0;  // largest |coordinate| of this thread's keys
 #pragma unroll
   for (int i = 0; i < COMPACT_PER_THREAD; ++i) {
     const int64_t sl = base + (int64_t)i * 256;
     keys[i] = sl < T ? tkeys[sl] : DEDUP_EMPTY;
-    mine += keys[i] != DEDUP_EMPTY;
+    if (keys[i] != DEDUP_EMPTY) {
+      ++mine;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) dev = max(dev, abs((int)((keys[i] >> (21 * c)) & 0x1fffff) - 1048576));
+    }
   }
+  dev = __reduce_max_sync(0xffffffffu, dev);
+  if (lane == 0 && dev > 0) atomicMax(maxdev, dev);
   unsigned incl = mine;  // inclusive warp scan
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -682,14 +693,24 @@ __global__ void __launch_bounds__(256) unique_compact_kernel(const uint64_t* tke
   }
 }
 
+// 63-bit keys -> the same order in 3 b bits: the fields of coordinates |c| <= m (2^b > 2 m).
+// An orbit's baselines use 10-14 of a field's 21 bits, so the radix sort takes 4-6 passes, not 8.
+__global__ void pack_keys_kernel(uint64_t* keys, int64_t n, int m, int b) {
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const uint64_t key = keys[k];
+  const uint64_t lo = 1048576 - m;
+  keys[k] = ((((key >> 42) & 0x1fffff) - lo) << (2 * b)) | ((((key >> 21) & 0x1fffff) - lo) << b) | ((key & 0x1fffff) - lo);
+}
+
 // sorted unique row indices -> their uvw, recomputed as the baselines kernel does
 __global__ void unique_emit_kernel(const uint32_t* idx, const int64_t* n, const float* pos, int64_t S, int nsat,
                                    int ordered, double lambda, float2 scale, float* u, float* v, float* w) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= *n) return;
-  const int64_t r = idx[k];  // pair-major row q * S + g
-  const int64_t q = r / S;
-  const int64_t g = r - q * S;
+  const uint32_t r = idx[k];  // pair-major row q * S + g
+  const uint32_t q = r / (uint32_t)S;
+  const int64_t g = r - q * (uint32_t)S;
   int m, nn;
   pair_of((int)q, nsat, ordered, &m, &nn);
   const float* pm = pos + (g * nsat + m) * 3;
@@ -713,12 +734,32 @@ __global__ void dedup_emit_kernel(const uint32_t* idx, const int64_t* n, const f
   ou[k] = u[s]; ov[k] = v[s]; ow[k] = w[s];
 }
 
+// Device counters of a table pass, read back in one copy.
+struct DedupCounters {
+  int bad, overflow;  // keys out of range; a key found no slot
+  int maxdev, pad;    // largest |coordinate| among the unique keys
+  int64_t n;          // unique keys
+};
+
+// Sort n unique (key, row) pairs by key, k1/i1 -> k0/i0 (k1 is rewritten with shorter keys).
+static int sort_unique(uint64_t* k1, uint64_t* k0, uint32_t* i1, uint32_t* i0, int64_t n, int maxdev, void* cub_temp,
+                       size_t cub_bytes, cudaStream_t st) {
+  if (n <= 0) return VISS_OK;
+  int b = 1;
+  while ((1 << b) <= 2 * maxdev) ++b;
+  pack_keys_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(k1, n, maxdev, b);
+  VISS_LAUNCH_CHECK("pack_keys_kernel");
+  // unique keys: the sort's stability does not matter
+  VISS_CUDA(cub::DeviceRadixSort::SortPairs(cub_temp, cub_bytes, k1, k0, i1, i0, n, 0, 3 * b, st));
+  return VISS_OK;
+}
+
 struct DedupPlan {
   uint64_t *k0 = nullptr, *k1 = nullptr;
   uint32_t *i0 = nullptr, *i1 = nullptr;
   float *tu = nullptr, *tv = nullptr, *tw = nullptr;
   int* flag = nullptr;
-  int* bad = nullptr;
+  DedupCounters* cnt = nullptr;
   int64_t* nsel = nullptr;
   void* cub = nullptr;
   size_t cub_bytes = 0, bytes = 0;
@@ -728,7 +769,7 @@ struct DedupPlan {
     i0 = c.take<uint32_t>(K); i1 = c.take<uint32_t>(K);
     tu = c.take<float>(K); tv = c.take<float>(K); tw = c.take<float>(K);
     flag = c.take<int>(K);
-    bad = c.take<int>(4);
+    cnt = c.take<DedupCounters>(1);
     nsel = c.take<int64_t>(4);
     size_t a = 0, b = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, a, (uint64_t*)nullptr, (uint64_t*)nullptr, (uint32_t*)nullptr,
@@ -754,8 +795,7 @@ struct UniquePlan {
   int64_t T = 0;
   uint64_t *tkeys = nullptr, *k1 = nullptr;
   uint32_t *tidx = nullptr, *i1 = nullptr;
-  int* bad = nullptr;
-  int64_t* nsel = nullptr;
+  DedupCounters* cnt = nullptr;
   void* cub = nullptr;
   size_t cub_bytes = 0, bytes = 0;
   void layout(void* ws, int64_t K) {
@@ -764,8 +804,7 @@ struct UniquePlan {
     Carver c(ws);
     tkeys = c.take<uint64_t>(T); k1 = c.take<uint64_t>(T);
     tidx = c.take<uint32_t>(T); i1 = c.take<uint32_t>(T);
-    bad = c.take<int>(4);
-    nsel = c.take<int64_t>(4);
+    cnt = c.take<DedupCounters>(1);
     cub::DeviceRadixSort::SortPairs(nullptr, cub_bytes, (uint64_t*)nullptr, (uint64_t*)nullptr, (uint32_t*)nullptr,
                                     (uint32_t*)nullptr, T, 0, 63);
     cub = c.take<char>(cub_bytes);
@@ -898,7 +937,7 @@ int viss_dedup_uvw(float* u, float* v, float* w, int64_t K, int64_t* count_out, 
   if (reinterpret_cast<uintptr_t>(workspace) & 255) return fail(VISS_ERR_WORKSPACE, "workspace misaligned");
   p.layout(workspace, K);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  VISS_CUDA(cudaMemsetAsync(p.bad, 0, 4 * sizeof(int), st));
+  VISS_CUDA(cudaMemsetAsync(p.cnt, 0, sizeof(DedupCounters), st));
   const unsigned nb = (unsigned)((K + 255) / 256);
   // Hash pass first, in the sort path's buffers: a table of T slots (keys in k0,
   // first indices in i0; T <= K, the buffers' length), from 2^25 slots up to 2^28
@@ -910,25 +949,21 @@ int viss_dedup_uvw(float* u, float* v, float* w, int64_t K, int64_t* count_out, 
     if (T <= prev) break;
     dedup_table_init_kernel<<<(unsigned)((T + 255) / 256), 256, 0, st>>>(p.k0, p.i0, T);
     VISS_LAUNCH_CHECK("dedup_table_init_kernel");
-    dedup_hash_kernel<<<nb, 256, 0, st>>>(u, v, w, K, p.k0, p.i0, (uint64_t)(T - 1), p.bad, p.bad + 1);
+    dedup_hash_kernel<<<nb, 256, 0, st>>>(u, v, w, K, p.k0, p.i0, (uint64_t)(T - 1), &p.cnt->bad, &p.cnt->overflow);
     VISS_LAUNCH_CHECK("dedup_hash_kernel");
-    int hb[2] = {0, 0};
-    VISS_CUDA(cudaMemcpyAsync(hb, p.bad, sizeof(hb), cudaMemcpyDeviceToHost, st));
+    unique_compact_kernel<<<(unsigned)((T + COMPACT_SLOTS - 1) / COMPACT_SLOTS), 256, 0, st>>>(
+        p.k0, p.i0, T, p.k1, p.i1, (unsigned long long*)&p.cnt->n, &p.cnt->maxdev);
+    VISS_LAUNCH_CHECK("unique_compact_kernel");
+    DedupCounters h{};
+    VISS_CUDA(cudaMemcpyAsync(&h, p.cnt, sizeof(h), cudaMemcpyDeviceToHost, st));
     VISS_CUDA(cudaStreamSynchronize(st));
-    if (hb[0]) return fail(VISS_ERR_RANGE, "dedup needs integer-valued uvw with |x| < 2^20");
-    if (!hb[1]) {
-      VISS_CUDA(cudaMemsetAsync(p.nsel, 0, sizeof(int64_t), st));
-      unique_compact_kernel<<<(unsigned)((T + COMPACT_SLOTS - 1) / COMPACT_SLOTS), 256, 0, st>>>(
-          p.k0, p.i0, T, p.k1, p.i1, (unsigned long long*)p.nsel);
-      VISS_LAUNCH_CHECK("unique_compact_kernel");
-      int64_t n = 0;
-      VISS_CUDA(cudaMemcpyAsync(&n, p.nsel, sizeof(n), cudaMemcpyDeviceToHost, st));
-      VISS_CUDA(cudaStreamSynchronize(st));
-      // unique keys: the sort's stability does not matter
-      size_t cb = p.cub_bytes;
-      VISS_CUDA(cub::DeviceRadixSort::SortPairs(p.cub, cb, p.k1, p.k0, p.i1, p.i0, n, 0, 63, st));
+    if (h.bad) return fail(VISS_ERR_RANGE, "dedup needs integer-valued uvw with |x| < 2^20");
+    if (!h.overflow) {
+      const int64_t n = h.n;
+      int rc = sort_unique(p.k1, p.k0, p.i1, p.i0, n, h.maxdev, p.cub, p.cub_bytes, st);
+      if (rc) return rc;
       if (n > 0) {
-        dedup_emit_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(p.i0, p.nsel, u, v, w, p.tu, p.tv, p.tw);
+        dedup_emit_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(p.i0, &p.cnt->n, u, v, w, p.tu, p.tv, p.tw);
         VISS_LAUNCH_CHECK("dedup_emit_kernel");
         VISS_CUDA(cudaMemcpyAsync(u, p.tu, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
         VISS_CUDA(cudaMemcpyAsync(v, p.tv, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
@@ -938,10 +973,10 @@ int viss_dedup_uvw(float* u, float* v, float* w, int64_t K, int64_t* count_out, 
       *count_out = n;
       return VISS_OK;
     }
-    VISS_CUDA(cudaMemsetAsync(p.bad, 0, 4 * sizeof(int), st));
+    VISS_CUDA(cudaMemsetAsync(p.cnt, 0, sizeof(DedupCounters), st));
     if (T >= ((int64_t)1 << 28)) break;
   }
-  dedup_keys_kernel<<<nb, 256, 0, st>>>(u, v, w, K, p.k0, p.i0, p.bad);
+  dedup_keys_kernel<<<nb, 256, 0, st>>>(u, v, w, K, p.k0, p.i0, &p.cnt->bad);
   VISS_LAUNCH_CHECK("dedup_keys_kernel");
   // stable radix sort: among equal keys the first input occurrence stays first
   size_t cb = p.cub_bytes;
@@ -956,7 +991,7 @@ int viss_dedup_uvw(float* u, float* v, float* w, int64_t K, int64_t* count_out, 
   }
   int bad = 0;
   int64_t cnt = 0;
-  VISS_CUDA(cudaMemcpyAsync(&bad, p.bad, sizeof(int), cudaMemcpyDeviceToHost, st));
+  VISS_CUDA(cudaMemcpyAsync(&bad, &p.cnt->bad, sizeof(int), cudaMemcpyDeviceToHost, st));
   VISS_CUDA(cudaMemcpyAsync(&cnt, p.nsel, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   VISS_CUDA(cudaStreamSynchronize(st));
   if (bad) return fail(VISS_ERR_RANGE, "dedup needs integer-valued uvw with |x| < 2^20");
@@ -992,40 +1027,47 @@ int viss_unique_uvw(const float* pos, int64_t S, int32_t nsat, int ordered, doub
   p.layout(workspace, K);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const float2 scale = scale_pair(lambda_m);
-  const int64_t threads = (S + UNIQUE_RUN - 1) / UNIQUE_RUN * (nsat * (nsat - 1) / 2);
-  // a table of 2^25 slots first (the few tens of millions of unique rows of an
-  // orbit campaign), the workspace's full table if that one fills
-  int64_t n = 0;
-  for (int64_t T = p.T < ((int64_t)1 << 25) ? p.T : ((int64_t)1 << 25);; T = p.T) {
-    VISS_CUDA(cudaMemsetAsync(p.bad, 0, 4 * sizeof(int), st));
-    VISS_CUDA(cudaMemsetAsync(p.nsel, 0, sizeof(int64_t), st));
+  const int nup = nsat * (nsat - 1) / 2;
+  // runs short enough for four waves of threads
+  int run = UNIQUE_RUN;
+  while (run > UNIQUE_RUN_MIN && S / run * nup < (int64_t)device_sm_count() * UNIQUE_CTAS * 256 * 4) run >>= 1;
+  const int64_t threads = (S + run - 1) / run * nup;
+  // First a table for about one unique row in eight, between 2^22 slots (50 MB: it stays in
+  // L2, 403,200 snapshots: initialising, inserting and compacting 941 -> 226 us against 2^25
+  // slots) and 2^25 (an orbit campaign's few tens of millions of unique rows), larger
+  // ones while it fills, up to the workspace's.
+  int64_t T = (int64_t)1 << 22;
+  while (T < ((int64_t)1 << 25) && T < K / 8) T <<= 1;
+  if (T > p.T) T = p.T;
+  DedupCounters h{};
+  for (;; T = T << 3 < p.T ? T << 3 : p.T) {
+    VISS_CUDA(cudaMemsetAsync(p.cnt, 0, sizeof(DedupCounters), st));
     dedup_table_init_kernel<<<(unsigned)((T + 255) / 256), 256, 0, st>>>(p.tkeys, p.tidx, T);
     VISS_LAUNCH_CHECK("dedup_table_init_kernel");
     unique_insert_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(
-        pos, S, nsat, ordered, npairs, lambda_m, scale, p.tkeys, p.tidx, (uint64_t)(T - 1), p.bad, p.bad + 1);
+        pos, S, nsat, ordered, run, lambda_m, scale, p.tkeys, p.tidx, (uint64_t)(T - 1), &p.cnt->bad, &p.cnt->overflow);
     VISS_LAUNCH_CHECK("unique_insert_kernel");
     unique_compact_kernel<<<(unsigned)((T + COMPACT_SLOTS - 1) / COMPACT_SLOTS), 256, 0, st>>>(
-        p.tkeys, p.tidx, T, p.k1, p.i1, (unsigned long long*)p.nsel);
+        p.tkeys, p.tidx, T, p.k1, p.i1, (unsigned long long*)&p.cnt->n, &p.cnt->maxdev);
     VISS_LAUNCH_CHECK("unique_compact_kernel");
-    int hb[2] = {0, 0};
-    VISS_CUDA(cudaMemcpyAsync(hb, p.bad, sizeof(hb), cudaMemcpyDeviceToHost, st));
-    VISS_CUDA(cudaMemcpyAsync(&n, p.nsel, sizeof(n), cudaMemcpyDeviceToHost, st));
+    VISS_CUDA(cudaMemcpyAsync(&h, p.cnt, sizeof(h), cudaMemcpyDeviceToHost, st));
     VISS_CUDA(cudaStreamSynchronize(st));
-    if (hb[0]) return fail(VISS_ERR_RANGE, "uvw beyond |x| < 2^20 cannot be keyed");
-    if (!hb[1]) break;
+    if (h.bad) return fail(VISS_ERR_RANGE, "uvw beyond |x| < 2^20 cannot be keyed");
+    if (!h.overflow) break;
     if (T == p.T)
       return fail(VISS_ERR_RANGE, "more unique uvw than the table holds: use viss_baseline_uvw + viss_dedup_uvw");
   }
+  const int64_t n = h.n;
   *count_out = n;
   if (n > capacity) {
     if (capacity == 0) return VISS_OK;  // count only
     return fail(VISS_ERR_RANGE, "capacity below the unique count (in *count_out)");
   }
   // unique keys, sorted with their first rows back into the table's buffers
-  size_t cb = p.cub_bytes;
-  VISS_CUDA(cub::DeviceRadixSort::SortPairs(p.cub, cb, p.k1, p.tkeys, p.i1, p.tidx, n, 0, 63, st));
+  int rc = sort_unique(p.k1, p.tkeys, p.i1, p.tidx, n, h.maxdev, p.cub, p.cub_bytes, st);
+  if (rc) return rc;
   if (n > 0) {
-    unique_emit_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(p.tidx, p.nsel, pos, S, nsat, ordered,
+    unique_emit_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(p.tidx, &p.cnt->n, pos, S, nsat, ordered,
                                                                     lambda_m, scale, u, v, w);
     VISS_LAUNCH_CHECK("unique_emit_kernel");
   }
