@@ -418,25 +418,29 @@ int launch_recon_fast(const ReconParams& p, int ctas_per_sm, bool comp, cudaStre
   return VISS_OK;
 }
 
-// F[c] = norm_c * -(sum of channel c's partial slots), slots summed in order in double.
-__global__ void recon_reduce_kernel(const RecReduceParams p) {
-  const int64_t pos = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// (s + e) * f, rounded once (but for the last bits of e)
+__device__ __forceinline__ float pair_times(const FloatPair& v, float f) {
+  const float h = __fmul_rn(v.s, f);
+  return h + __fmaf_rn(v.e, f, __fmaf_rn(v.s, f, -h));
+}
+
+// F[c] = norm_c * -(sum of channel c's partial slots), slots summed in a fixed order.
+// 10 MHz (256 slots x 196,608 pixels, 400 MB): 262 -> 48 us.
+__global__ void __launch_bounds__(32 * RED_GROUPS) recon_reduce_kernel(const RecReduceParams p) {
+  const int64_t pos = (int64_t)blockIdx.x * 32 + (threadIdx.x & 31);
   const int c = blockIdx.y;
-  if (pos >= p.J || p.nslot[c] == 0) return;
-  double sr = 0.0, si = 0.0;
-  for (int s = 0; s < p.nslot[c]; ++s) {
-    const float2 v = p.partial[(int64_t)(p.slot0[c] + s) * p.J + pos];
-    sr += v.x;
-    si += v.y;
+  if (p.nslot[c] == 0) return;
+  FloatPair re, im;
+  reduce_partials(p.partial + (int64_t)p.slot0[c] * p.J + pos, p.nslot[c], p.J, pos < p.J, re, im);
+  if (threadIdx.x < 32 && pos < p.J) {
+    const int64_t j = p.perm ? (int64_t)p.perm[pos] : pos;
+    p.out[(int64_t)c * p.J + j] = make_float2(pair_times(re, -p.norm[c]), pair_times(im, -p.norm[c]));
   }
-  const int64_t j = p.perm ? (int64_t)p.perm[pos] : pos;
-  const double norm = p.norm[c];
-  p.out[(int64_t)c * p.J + j] = make_float2((float)(-sr * norm), (float)(-si * norm));
 }
 
 int launch_recon_reduce(const RecReduceParams& p, cudaStream_t st) {
   if (p.J <= 0 || p.nch <= 0) return VISS_OK;
-  recon_reduce_kernel<<<dim3((unsigned)((p.J + 255) / 256), (unsigned)p.nch), 256, 0, st>>>(p);
+  recon_reduce_kernel<<<dim3((unsigned)((p.J + 31) / 32), (unsigned)p.nch), 32 * RED_GROUPS, 0, st>>>(p);
   VISS_LAUNCH_CHECK("recon_reduce_kernel");
   return VISS_OK;
 }

@@ -496,21 +496,18 @@ int launch_vis_fast(const VisParams& p, int ctas_per_sm, bool comp, cudaStream_t
   return VISS_OK;
 }
 
-__global__ void vis_reduce_kernel(const float2* __restrict__ part, int nsplit, int64_t K, float2* out) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= K) return;
-  double sr = 0.0, si = 0.0;
-  for (int s = 0; s < nsplit; ++s) {
-    const float2 v = part[(int64_t)s * K + k];
-    sr += v.x;
-    si += v.y;
-  }
-  out[k] = make_float2((float)-sr, (float)si);
+// 10 MHz (17 chunks x 1.8M rows, 250 MB): 266 -> 100 us.
+__global__ void __launch_bounds__(32 * RED_GROUPS) vis_reduce_kernel(const float2* __restrict__ part, int nsplit, int64_t K,
+                                                                     float2* out) {
+  const int64_t k = (int64_t)blockIdx.x * 32 + (threadIdx.x & 31);
+  FloatPair re, im;
+  reduce_partials(part + k, nsplit, K, k < K, re, im);
+  if (threadIdx.x < 32 && k < K) out[k] = make_float2(-(re.s + re.e), im.s + im.e);
 }
 
 int launch_vis_reduce(const float2* partial, int nsplit, int64_t K, float2* out, cudaStream_t st) {
   if (K <= 0) return VISS_OK;
-  vis_reduce_kernel<<<(unsigned)((K + 255) / 256), 256, 0, st>>>(partial, nsplit, K, out);
+  vis_reduce_kernel<<<(unsigned)((K + 31) / 32), 32 * RED_GROUPS, 0, st>>>(partial, nsplit, K, out);
   VISS_LAUNCH_CHECK("vis_reduce_kernel");
   return VISS_OK;
 }

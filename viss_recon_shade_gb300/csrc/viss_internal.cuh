@@ -71,6 +71,9 @@ constexpr int REC_THREADS = 256;
 constexpr int REC_TJ = 4;                 // pixels per thread
 constexpr int REC_PIX = REC_THREADS * REC_TJ;
 constexpr int REC_Q = 256;                // visibilities per shared-memory tile
+// Sums of work items' partial results: a block adds the partials of 32 consecutive outputs,
+// RED_GROUPS warps side by side, each every RED_GROUPS-th partial.
+constexpr int RED_GROUPS = 8;
 
 // Resident CTAs per SM the tiled kernels are compiled for (register budget
 // 65536 / (256 * n)).
@@ -146,6 +149,53 @@ __device__ __forceinline__ bool geo_occluded_exact(float sx_, float sy_, float s
   const double c = __dsub_rn(pp, __dmul_rn(R, R));
   const double disc = __dsub_rn(__dmul_rn(b, b), __dmul_rn(a, c));
   return (b < 0.0) && (disc > 0.0);
+}
+
+// A sum in a float pair (s + e is the sum to ~2^-46): Knuth's two-sum per addend.
+struct FloatPair {
+  float s = 0.f, e = 0.f;
+  __device__ __forceinline__ void add(float x) {
+    const float t = __fadd_rn(s, x), b = __fsub_rn(t, s);
+    e = __fadd_rn(e, __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(x, b)));
+    s = t;
+  }
+};
+
+// The sum over s < n of part[s * stride] (s in a fixed order: this warp's every RED_GROUPS-th,
+// then the warps' sums in order); valid in warp 0.  Float pairs, not double: at 2 FP64 lanes
+// per SM and clock the conversions and additions of double sums took five times the HBM reads
+// of the partials (10 MHz vis: 31M partials, 266 us).  Four loads are in flight per thread.
+__device__ __forceinline__ void reduce_partials(const float2* part, int n, int64_t stride, bool live, FloatPair& re,
+                                                FloatPair& im) {
+  __shared__ float4 sums[RED_GROUPS][32];
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+  if (live) {
+    int s = g;
+    for (; s + 3 * RED_GROUPS < n; s += 4 * RED_GROUPS) {
+      float2 v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = __ldcs(part + (int64_t)(s + i * RED_GROUPS) * stride);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) { re.add(v[i].x); im.add(v[i].y); }
+    }
+    for (; s < n; s += RED_GROUPS) {
+      const float2 v = __ldcs(part + (int64_t)s * stride);
+      re.add(v.x);
+      im.add(v.y);
+    }
+  }
+  sums[g][lane] = make_float4(re.s, re.e, im.s, im.e);
+  __syncthreads();
+  if (g == 0) {
+#pragma unroll
+    for (int i = 1; i < RED_GROUPS; ++i) {
+      const float4 v = sums[i][lane];
+      re.add(v.x);
+      re.e += v.y;
+      im.add(v.z);
+      im.e += v.w;
+    }
+  }
 }
 
 // -------------------------------------------------------- kernel params
