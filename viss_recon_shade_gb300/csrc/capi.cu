@@ -170,6 +170,16 @@ static void plan_vis(VisPlan& p, const viss_dft_cfg& cfg, const Batch& bt, int64
   if (nsplit > maxsplit) nsplit = maxsplit;
   if (nsplit < 1) nsplit = 1;
   p.jchunk = round_up((J + nsplit - 1) / nsplit, VIS_P);
+  // A small pass has fewer than 2 chunks of VIS_P pixels per CTA: shorter ones, down to
+  // VIS_MIN_CHUNK, so that every SM has work and the last wave is short (a power of two,
+  // so that a chunk stays within the VIS_P positions one REF range entry covers).  3,360 rows x
+  // 2,048 pixels: 93 -> 24 us; 28,672 x 12,288: geometric 197 (512 pixels), 185 (256), 206
+  // (128) us, REF windows 184 / 170 / 169 us.
+  if (tn.vis_split <= 0) {
+    int64_t chunk = VIS_P;
+    while (chunk > VIS_MIN_CHUNK && p.nrb * ((J + chunk - 1) / chunk) < 2 * slots) chunk >>= 1;
+    if (chunk < VIS_P) p.jchunk = chunk;
+  }
   if (p.jchunk <= 0) p.jchunk = VIS_P;
   p.nsplit = (int)((J + p.jchunk - 1) / p.jchunk);
   if (p.nsplit < 1) p.nsplit = 1;
@@ -234,13 +244,20 @@ struct RecPlan {
 // for ~rec_items work items (segment x pixel block) per resident CTA; at most
 // VISS_MAX_SEG segments.  Segments are ordered longest first.
 static void plan_segments(RecPlan& p, const Batch& bt, const Tuning& tn) {
-  constexpr int64_t unit = REC_Q;
+  int64_t unit = REC_Q;
   const int nch = bt.ch.nch;
   // items per CTA: many short segments balance blocks whose pixels the Moon hides for
   // different parts of the orbit (10 MHz recon: 4 items 191 ms, 8 176 ms, 32 167 ms, 64 165 ms)
   // resident CTAs: VISS_REC_MINB for the geometric kernel, one more for the others (recon.cu)
   const int64_t target = (tn.rec_items > 0 ? tn.rec_items : 64) * planned_ctas(tn, p.geo ? VISS_REC_MINB : VISS_REC_MINB + 1);
   int64_t L = p.npb > 0 ? (p.K * p.npb + target - 1) / target : p.K;
+  // A small pass has fewer than 4 segments of REC_Q rows per CTA: shorter ones, down to
+  // REC_MIN_ROWS, so that every SM has work.  3,360 rows x 2,048 pixels: 58 -> 20 us;
+  // 28,672 x 12,288: REF windows 256 rows 190 us, 128 rows 184 us, geometric 252 us either way.
+  if (tn.rec_items <= 0 && L < unit) {
+    while (unit > REC_MIN_ROWS && p.K * p.npb < 4 * (target / 64) * unit) unit >>= 1;
+    L = unit;
+  }
   L = round_up(L > unit ? L : unit, unit);
   auto count = [&](int64_t len) {
     int64_t n = 0;
@@ -250,7 +267,7 @@ static void plan_segments(RecPlan& p, const Batch& bt, const Tuning& tn) {
     }
     return n;
   };
-  while (count(L) > VISS_MAX_SEG) L = round_up(L + L / 4 + 1, unit);
+  while (count(L) > VISS_MAX_SEG) L = round_up(L + (L > 256 ? L / 4 : 0) + 1, unit);
   struct Seg { int64_t lo, hi; int ch, idx; };
   Seg segs[VISS_MAX_SEG];
   int ns = 0, slots = 0;

@@ -71,6 +71,8 @@ constexpr int REC_THREADS = 256;
 constexpr int REC_TJ = 4;                 // pixels per thread
 constexpr int REC_PIX = REC_THREADS * REC_TJ;
 constexpr int REC_Q = 256;                // visibilities per shared-memory tile
+constexpr int VIS_MIN_CHUNK = 32;         // least pixels of a vis work item
+constexpr int REC_MIN_ROWS = 32;          // least rows of a recon work item
 // Sums of work items' partial results: a block adds the partials of 32 consecutive outputs,
 // RED_GROUPS warps side by side, each every RED_GROUPS-th partial.
 constexpr int RED_GROUPS = 8;
