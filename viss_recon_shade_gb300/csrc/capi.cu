@@ -393,7 +393,7 @@ int vis_dft_impl(const viss_dft_cfg& cfg, const double scale[3], const float dlm
   VISS_CUDA(cudaMemsetAsync(p.flags, 0, FLAG_WORDS * sizeof(int), st));
   if (p.plain) {
     // the reference's form: one launch per channel
-    if (p.geo && (rc = launch_prep_satdir(geo->sat_pos, p.nsd, cfg.moon_radius_km, p.satdir, st))) return rc;
+    if (p.geo && (rc = launch_prep_satellites(geo->sat_pos, geo->S, geo->nsat, cfg.moon_radius_km, p.satdir, nullptr, st))) return rc;
     for (int c = 0; c < bt.ch.nch; ++c) {
       const int64_t r0 = bt.ch.row_off[c], r1 = bt.ch.row_off[c + 1];
       if (r1 == r0) continue;
@@ -429,7 +429,7 @@ int vis_dft_impl(const viss_dft_cfg& cfg, const double scale[3], const float dlm
   ra.flags = p.flags;
   if ((rc = launch_prep_rows(ra, false, st))) return rc;
   if (p.geo) {
-    if ((rc = launch_prep_satdir(geo->sat_pos, p.nsd, cfg.moon_radius_km, p.satdir, st))) return rc;
+    if ((rc = launch_prep_satellites(geo->sat_pos, geo->S, geo->nsat, cfg.moon_radius_km, p.satdir, nullptr, st))) return rc;
     if ((rc = launch_prep_rowblock_cones(p.rowsat, p.satdir, bt.ch, p.nrb, p.cones, st))) return rc;
   }
   VisParams vp{};
@@ -479,7 +479,7 @@ int recon_impl(const viss_dft_cfg& cfg, const double scale[3], const float dlmn[
       VISS_CUDA(cudaMemsetAsync(F2 + (int64_t)c * sky.J, 0, sizeof(float2) * (size_t)sky.J, st));
   if (p.plain) {
     // the reference's form: one launch per channel
-    if (p.geo && (rc = launch_prep_satdir(geo->sat_pos, p.nsd, cfg.moon_radius_km, p.satdir, st))) return rc;
+    if (p.geo && (rc = launch_prep_satellites(geo->sat_pos, geo->S, geo->nsat, cfg.moon_radius_km, p.satdir, nullptr, st))) return rc;
     for (int c = 0; c < bt.ch.nch; ++c) {
       const int64_t r0 = bt.ch.row_off[c], r1 = bt.ch.row_off[c + 1];
       if (r1 == r0) continue;
@@ -516,7 +516,7 @@ int recon_impl(const viss_dft_cfg& cfg, const double scale[3], const float dlmn[
   pa.sl = scale[0]; pa.sm = scale[1]; pa.sn = scale[2]; pa.n_offset = cfg.n_offset;
   pa.res = cfg.res; pa.trunc = 0;
   pa.rec0 = p.pix0; pa.rec1 = p.pix1; pa.lo = p.plo; pa.geo = p.pgeo; pa.qr = p.pqr;
-  if ((rc = launch_prep_pixels(pa, st))) return rc;
+  if ((rc = p.geo ? launch_prep_pixels_caps(pa, p.bcones, p.wcones, st) : launch_prep_pixels(pa, st))) return rc;
   RowPrepArgs ra{};
   ra.u = vis.u; ra.v = vis.v; ra.w = vis.w; ra.wgt = vis.wgt; ra.V = V;
   ra.shade = ratio_arrays ? nullptr : vis.shade;
@@ -534,10 +534,7 @@ int recon_impl(const viss_dft_cfg& cfg, const double scale[3], const float dlmn[
       return rc;
   }
   if (p.geo) {
-    if ((rc = launch_prep_satdir(geo->sat_pos, p.nsd, cfg.moon_radius_km, p.satdir, st))) return rc;
-    if ((rc = launch_prep_snapshot_cones(p.satdir, geo->S, geo->nsat, p.scones, st))) return rc;
-    if ((rc = launch_prep_block_cones(p.pgeo, sky.J, REC_PIX, p.npb, p.bcones, st))) return rc;
-    if ((rc = launch_prep_block_cones(p.pgeo, sky.J, 32 * REC_TJ, p.npb * (REC_THREADS / 32), p.wcones, st)))
+    if ((rc = launch_prep_satellites(geo->sat_pos, geo->S, geo->nsat, cfg.moon_radius_km, p.satdir, p.scones, st)))
       return rc;
   }
   ReconParams rp{};

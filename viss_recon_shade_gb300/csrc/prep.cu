@@ -12,16 +12,14 @@ namespace viss {
 // wavelength, evaluated in double from the float inputs.
 // Records are written at position `pos`; with a permutation the pixel at pos
 // is perm[pos] (records keep the original index in rec1.w / geo.w).
-__global__ void prep_pixels_kernel(PixPrepArgs a) {
-  const int64_t pos = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (pos >= a.Jpad) return;
+__device__ __forceinline__ float4 prep_pixel(const PixPrepArgs& a, int64_t pos) {
   if (pos >= a.J) {
     a.rec0[pos] = make_int4(0, 0, 0, 0);
     if (a.rec1) a.rec1[pos] = make_int4(0, 0, 0, (int)pos);
     if (a.lo) a.lo[pos] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (a.geo) a.geo[pos] = make_float4(0.f, 0.f, 0.f, __int_as_float((int)pos));
     if (a.qr) a.qr[pos] = make_int2(-1, -1);
-    return;
+    return make_float4(0.f, 0.f, 0.f, 0.f);
   }
   const int64_t j = a.perm ? (int64_t)a.perm[pos] : pos;
   const double x = a.sl * (double)a.l[j];
@@ -45,11 +43,13 @@ __global__ void prep_pixels_kernel(PixPrepArgs a) {
     a.lo[pos] = make_float4((float)((xa - rint(xa)) / sc), (float)((ya - rint(ya)) / sc),
                           (float)((za - rint(za)) / sc), 0.f);
   }
+  float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
   if (a.geo) {
     const double gx = a.l[j], gy = a.m[j], gz = a.n[j];
-    const double nn = sqrt(gx * gx + gy * gy + gz * gz);
-    const double inv = nn > 0 ? 1.0 / nn : 0.0;
-    a.geo[pos] = make_float4((float)(gx * inv), (float)(gy * inv), (float)(gz * inv), __int_as_float((int)j));
+    const double nn = gx * gx + gy * gy + gz * gz;
+    const double inv = nn > 0 ? rsqrt(nn) : 0.0;
+    g = make_float4((float)(gx * inv), (float)(gy * inv), (float)(gz * inv), __int_as_float((int)j));
+    a.geo[pos] = g;
   }
   if (a.qr) {
     const int res = a.res > 0 ? a.res : 1;
@@ -58,6 +58,100 @@ __global__ void prep_pixels_kernel(PixPrepArgs a) {
     if (r < 0) { r += res; --q; }  // floor division for negative indices
     a.qr[pos] = make_int2((int)q, (int)r);
   }
+  return g;
+}
+
+__global__ void prep_pixels_kernel(const PixPrepArgs a) {
+  const int64_t pos = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (pos < a.Jpad) prep_pixel(a, pos);
+}
+
+__device__ __forceinline__ float warp_sum(float x) {
+  for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+__device__ __forceinline__ float warp_max(float x) {
+  for (int o = 16; o; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
+  return x;
+}
+__device__ __forceinline__ float warp_min(float x) {
+  for (int o = 16; o; o >>= 1) x = fminf(x, __shfl_xor_sync(0xffffffffu, x, o));
+  return x;
+}
+__device__ __forceinline__ float chord2(const float4& a, const float4& g) {  // |a - g|^2
+  const float dx = g.x - a.x, dy = g.y - a.y, dz = g.z - a.z;
+  return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+}
+
+// Bounding cap of unit vectors: their normalised sum as axis, and the angle r of their largest
+// distance c from it, c = 2 sin(r / 2) (a chord keeps its relative accuracy in FP32 where a
+// cosine near 1 does not), widened by 2e-6 against the rounding of both.  {axis, cos r},
+// {sin r}; cos r = -2 without an axis.
+__device__ __forceinline__ float4 cap_axis(float sx, float sy, float sz) {
+  const float nn = sqrtf(fmaf(sx, sx, fmaf(sy, sy, sz * sz)));
+  return nn > 1e-3f ? make_float4(sx / nn, sy / nn, sz / nn, 1.f) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+__device__ __forceinline__ void cap_write(const float4& axis, float c2, float4* out) {
+  float cr = -2.f, sr = 1.f;
+  if (axis.w != 0.f && c2 < 3.999f) {
+    const float r = 2.f * asinf(0.5f * sqrtf(c2)) + 2e-6f;
+    cr = cosf(r);
+    sr = sinf(r);
+  }
+  out[0] = make_float4(axis.x, axis.y, axis.z, cr);
+  out[1] = make_float4(sr, 0.f, 0.f, 0.f);
+}
+
+// The records and, on the way, the caps of each warp's patch of 32 * REC_TJ positions and of each
+// block of REC_PIX: one launch and no second read of the directions (two cap kernels with
+// FP64 cosines and arc cosines took 22 us beside 5 us of records on 2,048-12,288 pixels).
+__global__ void __launch_bounds__(REC_THREADS) prep_pixels_caps_kernel(const PixPrepArgs a, float4* bcaps, float4* wcaps) {
+  __shared__ float4 s_sum[REC_THREADS / 32];
+  __shared__ float s_c2[REC_THREADS / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t p0 = (int64_t)blockIdx.x * REC_PIX + warp * 32 * REC_TJ + lane;
+  float4 g[REC_TJ];
+  float sx = 0.f, sy = 0.f, sz = 0.f;
+#pragma unroll
+  for (int i = 0; i < REC_TJ; ++i) {
+    g[i] = prep_pixel(a, p0 + 32 * i);  // zero past the last pixel
+    sx += g[i].x; sy += g[i].y; sz += g[i].z;
+  }
+  sx = warp_sum(sx); sy = warp_sum(sy); sz = warp_sum(sz);
+  const float4 wa = cap_axis(sx, sy, sz);
+  float c2 = 0.f;
+#pragma unroll
+  for (int i = 0; i < REC_TJ; ++i)
+    if (p0 + 32 * i < a.J) c2 = fmaxf(c2, chord2(wa, g[i]));
+  c2 = warp_max(c2);
+  if (lane == 0) {
+    cap_write(wa, c2, wcaps + 2 * ((int64_t)blockIdx.x * (REC_THREADS / 32) + warp));
+    s_sum[warp] = make_float4(sx, sy, sz, 0.f);
+  }
+  __syncthreads();
+  sx = sy = sz = 0.f;
+#pragma unroll
+  for (int w = 0; w < REC_THREADS / 32; ++w) { sx += s_sum[w].x; sy += s_sum[w].y; sz += s_sum[w].z; }
+  const float4 ba = cap_axis(sx, sy, sz);
+  c2 = 0.f;
+#pragma unroll
+  for (int i = 0; i < REC_TJ; ++i)
+    if (p0 + 32 * i < a.J) c2 = fmaxf(c2, chord2(ba, g[i]));
+  c2 = warp_max(c2);
+  if (lane == 0) s_c2[warp] = c2;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < REC_THREADS / 32; ++w) c2 = fmaxf(c2, s_c2[w]);
+    cap_write(ba, c2, bcaps + 2 * blockIdx.x);
+  }
+}
+
+int launch_prep_pixels_caps(const PixPrepArgs& a, float4* bcaps, float4* wcaps, cudaStream_t st) {
+  if (a.Jpad <= 0) return VISS_OK;
+  prep_pixels_caps_kernel<<<(unsigned)(a.Jpad / REC_PIX), REC_THREADS, 0, st>>>(a, bcaps, wcaps);
+  VISS_LAUNCH_CHECK("prep_pixels_caps_kernel");
+  return VISS_OK;
 }
 
 // {min, max} of widx over each run of VIS_P positions (the fine indices a vis
@@ -258,24 +352,13 @@ __global__ void prep_recon_ratios_kernel(const float* thetaP0, const float* phiP
 // seen from the satellite.  Occluded <=> s_hat . p_hat < -cos(alpha).  A
 // satellite inside the sphere (|p| <= R) gets cos(alpha) = 0 (occluded <=> s.p < 0),
 // which is what the exact predicate gives there.
-__global__ void prep_satdir_kernel(const float* pos, int64_t nsd, double R, float4* satdir) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nsd) return;
-  const double px = pos[3 * i], py = pos[3 * i + 1], pz = pos[3 * i + 2];
-  const double r = sqrt(px * px + py * py + pz * pz);
-  if (!(r > 0.0)) {
-    satdir[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    return;
-  }
-  const double ca = r > R ? sqrt(1.0 - (R / r) * (R / r)) : 0.0;
-  satdir[i] = make_float4((float)(px / r), (float)(py / r), (float)(pz / r), (float)ca);
-}
-
-int launch_prep_satdir(const float* sat_pos, int64_t nsd, double R, float4* satdir, cudaStream_t st) {
-  if (nsd <= 0) return VISS_OK;
-  prep_satdir_kernel<<<(unsigned)((nsd + 255) / 256), 256, 0, st>>>(sat_pos, nsd, R, satdir);
-  VISS_LAUNCH_CHECK("prep_satdir_kernel");
-  return VISS_OK;
+__device__ __forceinline__ float4 sat_direction(const float* pos, double R) {
+  const double px = pos[0], py = pos[1], pz = pos[2];
+  const double rr = px * px + py * py + pz * pz;
+  if (!(rr > 0.0)) return make_float4(0.f, 0.f, 0.f, 0.f);
+  const double inv = rsqrt(rr), q = R * inv;
+  const float ca = rr > R * R ? sqrtf((float)(1.0 - q * q)) : 0.f;
+  return make_float4((float)(px * inv), (float)(py * inv), (float)(pz * inv), ca);
 }
 
 // ------------------------------------------------------------- cones
@@ -286,116 +369,147 @@ int launch_prep_satdir(const float* sat_pos, int64_t nsd, double R, float4* satd
 // from every one.  cone[0] = {c, cos_occ}, cone[1] = {cos_vis, sin_occ, sin_vis, -}
 // (the sines of the two angles, 0 where the cosine is the 2 / -2 of "never").
 // Degenerate sets (a satellite at the origin) get cos_occ = 2, cos_vis = -2.
-// From the axis, the smallest cosine to it (mc) and the cone-angle range [a0, a1].
-__device__ void cone_write(const double* axis, double mc, double a0, double a1, bool degen, int64_t count,
-                           float4* out) {
-  const double eps = 1e-5;
+// In FP32: rho from the largest chord, alpha from the extreme cosines; each is good to 3e-7
+// rad, which the margins (1.2e-5 rad, 1.5e-6 in the cosine tested against) cover many times over.
+__device__ void cone_write(const float4& axis, float c2, float wmin, float wmax, bool degen, float4* out) {
+  const float eps = 1.2e-5f;
   float cos_occ = 2.f, cos_vis = -2.f, sin_occ = 0.f, sin_vis = 0.f;
-  if (!degen && count > 0) {
-    const double rho = acos(fmin(1.0, fmax(-1.0, mc)));
-    const double lo = a0 - rho - eps, hi = a1 + rho + eps;
-    if (lo > 0) { cos_occ = (float)cos(lo); sin_occ = (float)sin(lo); }
-    if (hi < kPi) { cos_vis = (float)cos(hi); sin_vis = (float)sin(hi); }
-    // widen by float rounding of the test s_hat . c
-    if (cos_occ <= 1.f) cos_occ = fminf(2.f, cos_occ + 1e-6f);
-    if (cos_vis >= -1.f) cos_vis = cos_vis - 1e-6f;
+  if (!degen) {
+    const float rho = 2.f * asinf(fminf(1.f, 0.5f * sqrtf(c2)));
+    const float lo = acosf(fminf(1.f, wmax)) - rho - eps, hi = acosf(fmaxf(-1.f, wmin)) + rho + eps;
+    if (lo > 0.f) { cos_occ = cosf(lo) + 1.5e-6f; sin_occ = sinf(lo); }
+    if (hi < 3.1415926f) { cos_vis = cosf(hi) - 1.5e-6f; sin_vis = sinf(hi); }
   }
-  out[0] = make_float4((float)axis[0], (float)axis[1], (float)axis[2], cos_occ);
+  out[0] = make_float4(axis.x, axis.y, axis.z, cos_occ);
   out[1] = make_float4(cos_vis, sin_occ, sin_vis, 0.f);
 }
-
-// Block-wide: one block per cone; members enumerated by `member(i)` -> satdir index.
-template <class Member>
-__device__ void cone_block(const float4* satdir, int64_t count, Member member, float4* out) {
-  __shared__ double red[4][32];
-  __shared__ double axis[3];
-  __shared__ int degen_s;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
-  if (tid == 0) degen_s = 0;
-  __syncthreads();
-  double sx = 0, sy = 0, sz = 0;
-  for (int64_t i = tid; i < count; i += blockDim.x) {
-    const float4 d = satdir[member(i)];
-    if (d.x == 0.f && d.y == 0.f && d.z == 0.f) { atomicOr(&degen_s, 1); continue; }
-    if (d.w == 0.f) atomicOr(&degen_s, 1);  // inside the sphere: no cone
-    sx -= d.x; sy -= d.y; sz -= d.z;
+// axis of a cone from the sum of -p_hat; no axis makes the set degenerate
+__device__ __forceinline__ float4 cone_axis(float sx, float sy, float sz, bool* degen) {
+  const float nn = sqrtf(fmaf(sx, sx, fmaf(sy, sy, sz * sz)));
+  if (!(nn > 1e-6f)) {
+    *degen = true;
+    return make_float4(0.f, 0.f, 1.f, 0.f);
   }
-  for (int o = 16; o; o >>= 1) {
+  return make_float4(sx / nn, sy / nn, sz / nn, 0.f);
+}
+__device__ __forceinline__ float4 minus(const float4& d) { return make_float4(-d.x, -d.y, -d.z, d.w); }
+// at the origin (no direction) or inside the sphere: no cone
+__device__ __forceinline__ bool no_cone(const float4& d) { return d.w == 0.f; }
+
+// Satellite directions and (cones != NULL) each snapshot's cone: a thread per satellite, G
+// lanes (a power of two >= nsat) per snapshot, so that a pass of a hundred snapshots is a few
+// short chains (one thread per snapshot with FP64 arc cosines took 20 us, the directions 5.5).
+__global__ void prep_satellites_kernel(const float* pos, int64_t S, int nsat, int G, double R, float4* satdir,
+                                       float4* cones) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t s = t / G;
+  const int i = (int)(t & (G - 1));
+  const bool live = s < S && i < nsat;
+  float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (live) {
+    d = sat_direction(pos + 3 * (s * nsat + i), R);
+    satdir[s * nsat + i] = d;
+  }
+  if (!cones) return;
+  float sx = -d.x, sy = -d.y, sz = -d.z;
+  float wmin = live ? d.w : 2.f, wmax = live ? d.w : -2.f;
+  int dg = live && no_cone(d);
+  for (int o = G >> 1; o; o >>= 1) {
     sx += __shfl_xor_sync(0xffffffffu, sx, o);
     sy += __shfl_xor_sync(0xffffffffu, sy, o);
     sz += __shfl_xor_sync(0xffffffffu, sz, o);
+    wmin = fminf(wmin, __shfl_xor_sync(0xffffffffu, wmin, o));
+    wmax = fmaxf(wmax, __shfl_xor_sync(0xffffffffu, wmax, o));
+    dg |= __shfl_xor_sync(0xffffffffu, dg, o);
   }
-  if (lane == 0) { red[0][wid] = sx; red[1][wid] = sy; red[2][wid] = sz; }
-  __syncthreads();
-  if (tid == 0) {
-    double a = 0, b = 0, c = 0;
-    for (int w = 0; w < nw; ++w) { a += red[0][w]; b += red[1][w]; c += red[2][w]; }
-    const double nn = sqrt(a * a + b * b + c * c);
-    axis[0] = nn > 0 ? a / nn : 0; axis[1] = nn > 0 ? b / nn : 0; axis[2] = nn > 0 ? c / nn : 1;
-    if (!(nn > 0)) degen_s = 1;
-  }
-  __syncthreads();
-  // rho (as min cos), alpha range
-  double mincos = 2.0, amin = 10.0, amax = -1.0;
-  for (int64_t i = tid; i < count; i += blockDim.x) {
-    const float4 d = satdir[member(i)];
-    const double c = -(axis[0] * d.x + axis[1] * d.y + axis[2] * d.z);
-    mincos = fmin(mincos, c);
-    const double al = acos(fmin(1.0, fmax(-1.0, (double)d.w)));
-    amin = fmin(amin, al);
-    amax = fmax(amax, al);
-  }
-  for (int o = 16; o; o >>= 1) {
-    mincos = fmin(mincos, __shfl_xor_sync(0xffffffffu, mincos, o));
-    amin = fmin(amin, __shfl_xor_sync(0xffffffffu, amin, o));
-    amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  }
-  __syncthreads();
-  if (lane == 0) { red[0][wid] = mincos; red[1][wid] = amin; red[2][wid] = amax; }
-  __syncthreads();
-  if (tid == 0) {
-    double mc = 2.0, a0 = 10.0, a1 = -1.0;
-    for (int w = 0; w < nw; ++w) { mc = fmin(mc, red[0][w]); a0 = fmin(a0, red[1][w]); a1 = fmax(a1, red[2][w]); }
-    cone_write(axis, mc, a0, a1, degen_s != 0, count, out);
-  }
+  bool degen = dg != 0;
+  const float4 axis = cone_axis(sx, sy, sz, &degen);
+  float c2 = live ? chord2(axis, minus(d)) : 0.f;
+  for (int o = G >> 1; o; o >>= 1) c2 = fmaxf(c2, __shfl_xor_sync(0xffffffffu, c2, o));
+  if (s < S && i == 0) cone_write(axis, c2, wmin, wmax, degen, cones + 2 * s);
 }
 
-struct RowMember {
-  const int* rowsat;
-  int64_t base;
-  __device__ int operator()(int64_t i) const {
-    const int p = rowsat[base + (i >> 1)];
-    return (i & 1) ? sat_gn(p) : sat_gm(p);
-  }
-};
+int launch_prep_satellites(const float* sat_pos, int64_t S, int nsat, double R, float4* satdir, float4* cones,
+                           cudaStream_t st) {
+  if (S <= 0 || nsat <= 0) return VISS_OK;
+  int G = 1;
+  while (G < nsat) G <<= 1;
+  const int64_t n = S * G;
+  prep_satellites_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(sat_pos, S, nsat, G, R, satdir, cones);
+  VISS_LAUNCH_CHECK("prep_satellites_kernel");
+  return VISS_OK;
+}
 
 // One cone per padded block of VIS_ROWS rows, over the block's real rows; the
 // sines in cone[1] (which the vis kernel does not use) are replaced by the range
 // of satellite indices those rows use (y: the first, z: how many, as int bits;
-// z = 0 for an empty block).
-__global__ void rowblock_cones_kernel(const int* rowsat, const float4* satdir, const ChannelRows ch, float4* cones) {
+// z = 0 for an empty block).  (With FP64 cosines and an FP64 arc cosine per satellite: 37 us
+// however few the blocks, 320 us for 1,792.)
+constexpr int CONE_THREADS = 256;
+__global__ void __launch_bounds__(CONE_THREADS) rowblock_cones_kernel(const int* rowsat, const float4* satdir,
+                                                                      const ChannelRows ch, float4* cones) {
+  constexpr int NW = CONE_THREADS / 32, PER = VIS_ROWS / CONE_THREADS;
+  __shared__ float red[NW][6];
+  __shared__ int redi[NW][3];
   const int64_t b = blockIdx.x;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int c = 0;
   while (c + 1 < ch.nch && b >= ch.rb_off[c + 1]) ++c;
   int64_t cnt = (ch.row_off[c + 1] - ch.row_off[c]) - (b - ch.rb_off[c]) * VIS_ROWS;
   if (cnt > VIS_ROWS) cnt = VIS_ROWS;
   if (cnt < 0) cnt = 0;
-  cone_block(satdir, 2 * cnt, RowMember{rowsat, b * VIS_ROWS}, cones + 2 * b);
-  __shared__ int rlo[32], rhi[32];
-  int lo = 0x7fffffff, hi = -1;
-  for (int64_t i = threadIdx.x; i < cnt; i += blockDim.x) {
-    const int pk = rowsat[b * VIS_ROWS + i];
-    lo = min(lo, min(sat_gm(pk), sat_gn(pk)));
-    hi = max(hi, max(sat_gm(pk), sat_gn(pk)));
+  int pk[PER];
+  float sx = 0.f, sy = 0.f, sz = 0.f, wmin = 2.f, wmax = -2.f;
+  int lo = 0x7fffffff, hi = -1, dg = 0;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int r = threadIdx.x + i * CONE_THREADS;
+    pk[i] = r < cnt ? rowsat[b * VIS_ROWS + r] : -1;
+    if (pk[i] == -1) continue;
+    const int gm = sat_gm(pk[i]), gn = sat_gn(pk[i]);
+    const float4 d1 = satdir[gm], d2 = satdir[gn];
+    sx -= d1.x + d2.x; sy -= d1.y + d2.y; sz -= d1.z + d2.z;
+    wmin = fminf(wmin, fminf(d1.w, d2.w));
+    wmax = fmaxf(wmax, fmaxf(d1.w, d2.w));
+    dg |= no_cone(d1) || no_cone(d2);
+    lo = min(lo, min(gm, gn));
+    hi = max(hi, max(gm, gn));
   }
-  for (int o = 16; o; o >>= 1) {
-    lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-    hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  sx = warp_sum(sx); sy = warp_sum(sy); sz = warp_sum(sz);
+  wmin = warp_min(wmin);
+  wmax = warp_max(wmax);
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  dg = __any_sync(0xffffffffu, dg);
+  if (lane == 0) {
+    red[wid][0] = sx; red[wid][1] = sy; red[wid][2] = sz; red[wid][3] = wmin; red[wid][4] = wmax;
+    redi[wid][0] = lo; redi[wid][1] = hi; redi[wid][2] = dg;
   }
-  if ((threadIdx.x & 31) == 0) { rlo[threadIdx.x >> 5] = lo; rhi[threadIdx.x >> 5] = hi; }
+  __syncthreads();
+  sx = sy = sz = 0.f;
+#pragma unroll
+  for (int w = 0; w < NW; ++w) {
+    sx += red[w][0]; sy += red[w][1]; sz += red[w][2];
+    wmin = fminf(wmin, red[w][3]);
+    wmax = fmaxf(wmax, red[w][4]);
+    lo = min(lo, redi[w][0]);
+    hi = max(hi, redi[w][1]);
+    dg |= redi[w][2];
+  }
+  bool degen = dg != 0 || cnt == 0;
+  const float4 axis = cone_axis(sx, sy, sz, &degen);
+  float c2 = 0.f;
+#pragma unroll
+  for (int i = 0; i < PER; ++i)
+    if (pk[i] != -1)
+      c2 = fmaxf(c2, fmaxf(chord2(axis, minus(satdir[sat_gm(pk[i])])), chord2(axis, minus(satdir[sat_gn(pk[i])]))));
+  c2 = warp_max(c2);
+  if (lane == 0) red[wid][5] = c2;
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) { lo = min(lo, rlo[w]); hi = max(hi, rhi[w]); }
+#pragma unroll
+    for (int w = 1; w < NW; ++w) c2 = fmaxf(c2, red[w][5]);
+    cone_write(axis, c2, wmin, wmax, degen, cones + 2 * b);
     cones[2 * b + 1].y = __int_as_float(hi >= lo ? lo : 0);
     cones[2 * b + 1].z = __int_as_float(hi >= lo ? hi - lo + 1 : 0);
   }
@@ -404,103 +518,8 @@ __global__ void rowblock_cones_kernel(const int* rowsat, const float4* satdir, c
 int launch_prep_rowblock_cones(const int* rowsat, const float4* satdir, const ChannelRows& ch, int64_t nblocks,
                                float4* cones, cudaStream_t st) {
   if (nblocks <= 0) return VISS_OK;
-  rowblock_cones_kernel<<<(unsigned)nblocks, 256, 0, st>>>(rowsat, satdir, ch, cones);
+  rowblock_cones_kernel<<<(unsigned)nblocks, CONE_THREADS, 0, st>>>(rowsat, satdir, ch, cones);
   VISS_LAUNCH_CHECK("rowblock_cones_kernel");
-  return VISS_OK;
-}
-
-// Bounding cone of each block of `block` consecutive sky positions (unit
-// directions in pgeo): axis = normalised mean, radius r = largest angle from it,
-// widened by 1e-6.  {axis, cos r}, {sin r}; cos r = -2 when the block has no axis.
-__global__ void block_cones_kernel(const float4* pgeo, int64_t J, int block, float4* cones) {
-  __shared__ double red[3][32];
-  __shared__ double axis[3];
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
-  const int64_t j0 = (int64_t)blockIdx.x * block;
-  int64_t j1 = j0 + block;
-  if (j1 > J) j1 = J;
-  double sx = 0, sy = 0, sz = 0;
-  for (int64_t j = j0 + tid; j < j1; j += blockDim.x) {
-    const float4 g = pgeo[j];
-    sx += g.x; sy += g.y; sz += g.z;
-  }
-  for (int o = 16; o; o >>= 1) {
-    sx += __shfl_xor_sync(0xffffffffu, sx, o);
-    sy += __shfl_xor_sync(0xffffffffu, sy, o);
-    sz += __shfl_xor_sync(0xffffffffu, sz, o);
-  }
-  if (lane == 0) { red[0][wid] = sx; red[1][wid] = sy; red[2][wid] = sz; }
-  __syncthreads();
-  if (tid == 0) {
-    double a = 0, b = 0, c = 0;
-    for (int w = 0; w < nw; ++w) { a += red[0][w]; b += red[1][w]; c += red[2][w]; }
-    const double nn = sqrt(a * a + b * b + c * c);
-    axis[0] = nn > 1e-3 ? a / nn : 0.0; axis[1] = nn > 1e-3 ? b / nn : 0.0; axis[2] = nn > 1e-3 ? c / nn : 0.0;
-  }
-  __syncthreads();
-  double mc = 2.0;
-  for (int64_t j = j0 + tid; j < j1; j += blockDim.x) {
-    const float4 g = pgeo[j];
-    mc = fmin(mc, axis[0] * g.x + axis[1] * g.y + axis[2] * g.z);
-  }
-  for (int o = 16; o; o >>= 1) mc = fmin(mc, __shfl_xor_sync(0xffffffffu, mc, o));
-  __syncthreads();
-  if (lane == 0) red[0][wid] = mc;
-  __syncthreads();
-  if (tid == 0) {
-    for (int w = 0; w < nw; ++w) mc = fmin(mc, red[0][w]);
-    const bool ok = (axis[0] != 0.0 || axis[1] != 0.0 || axis[2] != 0.0) && mc <= 1.0 && mc > -1.0;
-    double cr = -2.0, sr = 1.0;
-    if (ok) {
-      const double r = acos(fmin(1.0, mc)) + 1e-6;
-      cr = cos(r);
-      sr = sin(r);
-    }
-    cones[2 * blockIdx.x] = make_float4((float)axis[0], (float)axis[1], (float)axis[2], (float)cr);
-    cones[2 * blockIdx.x + 1] = make_float4((float)sr, 0.f, 0.f, 0.f);
-  }
-}
-
-int launch_prep_block_cones(const float4* pgeo, int64_t J, int block, int64_t nblocks, float4* cones,
-                            cudaStream_t st) {
-  if (nblocks <= 0) return VISS_OK;
-  block_cones_kernel<<<(unsigned)nblocks, 256, 0, st>>>(pgeo, J, block, cones);
-  VISS_LAUNCH_CHECK("block_cones_kernel");
-  return VISS_OK;
-}
-
-// One thread per snapshot (its nsat satellites in a loop): the bounds of
-// cone_block, without a block's reductions and serial tail per snapshot.
-__global__ void snapshot_cones_kernel(const float4* satdir, int64_t S, int nsat, float4* cones) {
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= S) return;
-  const float4* d0 = satdir + s * nsat;
-  bool degen = false;
-  double sx = 0, sy = 0, sz = 0;
-  for (int i = 0; i < nsat; ++i) {
-    const float4 d = d0[i];
-    if (d.x == 0.f && d.y == 0.f && d.z == 0.f) { degen = true; continue; }
-    if (d.w == 0.f) degen = true;  // inside the sphere: no cone
-    sx -= d.x; sy -= d.y; sz -= d.z;
-  }
-  const double nn = sqrt(sx * sx + sy * sy + sz * sz);
-  double axis[3] = {nn > 0 ? sx / nn : 0, nn > 0 ? sy / nn : 0, nn > 0 ? sz / nn : 1};
-  if (!(nn > 0)) degen = true;
-  double mc = 2.0, a0 = 10.0, a1 = -1.0;
-  for (int i = 0; i < nsat; ++i) {
-    const float4 d = d0[i];
-    mc = fmin(mc, -(axis[0] * d.x + axis[1] * d.y + axis[2] * d.z));
-    const double al = acos(fmin(1.0, fmax(-1.0, (double)d.w)));
-    a0 = fmin(a0, al);
-    a1 = fmax(a1, al);
-  }
-  cone_write(axis, mc, a0, a1, degen, nsat, cones + 2 * s);
-}
-
-int launch_prep_snapshot_cones(const float4* satdir, int64_t S, int nsat, float4* cones, cudaStream_t st) {
-  if (S <= 0) return VISS_OK;
-  snapshot_cones_kernel<<<(unsigned)((S + 127) / 128), 128, 0, st>>>(satdir, S, nsat, cones);
-  VISS_LAUNCH_CHECK("snapshot_cones_kernel");
   return VISS_OK;
 }
 

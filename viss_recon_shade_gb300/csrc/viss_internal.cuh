@@ -380,11 +380,11 @@ size_t pixel_order_scratch(int64_t J);
 int pixel_order(const float* l, const float* m, const float* n, int64_t J, void* scratch, size_t scratch_bytes,
                 int32_t* perm, cudaStream_t st);
 int launch_prep_rows(const RowPrepArgs& a, bool recon, cudaStream_t st);
-int launch_prep_satdir(const float* sat_pos, int64_t nsd, double R, float4* satdir, cudaStream_t st);
+int launch_prep_pixels_caps(const PixPrepArgs& a, float4* bcaps, float4* wcaps, cudaStream_t st);
+int launch_prep_satellites(const float* sat_pos, int64_t S, int nsat, double R, float4* satdir, float4* cones,
+                           cudaStream_t st);
 int launch_prep_rowblock_cones(const int* rowsat, const float4* satdir, const ChannelRows& ch, int64_t nblocks,
                                float4* cones, cudaStream_t st);
-int launch_prep_snapshot_cones(const float4* satdir, int64_t S, int nsat, float4* cones, cudaStream_t st);
-int launch_prep_block_cones(const float4* pgeo, int64_t J, int block, int64_t nblocks, float4* cones, cudaStream_t st);
 
 // Persistent launches: ctas_per_sm 0 = as many as fit.
 int launch_vis_fast(const VisParams& p, int ctas_per_sm, bool compensated, cudaStream_t st);
