@@ -362,6 +362,15 @@ static int check_ws(void* ws, size_t have, size_t need) {
 }
 
 // ------------------------------------------------------------------ passes
+// The phase scales of a pixel prep, and whether its FP32 form is exact (PixPrepArgs::pow2).
+static void set_scales(PixPrepArgs& a, const double scale[3], double n_offset) {
+  a.sl = scale[0]; a.sm = scale[1]; a.sn = scale[2]; a.n_offset = n_offset;
+  int e = 0;
+  const double off = scale[2] * n_offset * 4294967296.0;
+  a.pow2 = scale[0] == scale[1] && scale[0] == scale[2] && frexp(scale[0], &e) == 0.5 && e > -30 && off == rint(off);
+  a.off32 = a.pow2 ? (long long)off : 0;
+}
+
 static viss_vis_set channel_rows(const viss_vis_set& vis, int64_t r0, int64_t r1) {
   viss_vis_set c = vis;
   c.u = vis.u + r0; c.v = vis.v + r0; c.w = vis.w + r0;
@@ -412,7 +421,7 @@ int vis_dft_impl(const viss_dft_cfg& cfg, const double scale[3], const float dlm
   PixPrepArgs pa{};
   pa.l = sky.l; pa.m = sky.m; pa.n = sky.n; pa.bright = bt.bright ? nullptr : (map ? p.mbase : sky.bright);
   pa.J = sky.J; pa.Jpad = p.Jpad;
-  pa.sl = scale[0]; pa.sm = scale[1]; pa.sn = scale[2]; pa.n_offset = cfg.n_offset;
+  set_scales(pa, scale, cfg.n_offset);
   pa.res = cfg.res; pa.trunc = map ? 0 : cfg.trunc_brightness;  // the map's base brightness is truncated per member
   pa.rec0 = p.pix0; pa.rec1 = p.pix1; pa.lo = p.plo; pa.geo = p.pgeo; pa.qr = p.pqr;
   pa.widx = p.ref ? widx : nullptr;
@@ -513,7 +522,7 @@ int recon_impl(const viss_dft_cfg& cfg, const double scale[3], const float dlmn[
   pa.perm = p.perm;
   pa.l = sky.l; pa.m = sky.m; pa.n = sky.n; pa.bright = nullptr;
   pa.J = sky.J; pa.Jpad = p.Jpad;
-  pa.sl = scale[0]; pa.sm = scale[1]; pa.sn = scale[2]; pa.n_offset = cfg.n_offset;
+  set_scales(pa, scale, cfg.n_offset);
   pa.res = cfg.res; pa.trunc = 0;
   pa.rec0 = p.pix0; pa.rec1 = p.pix1; pa.lo = p.plo; pa.geo = p.pgeo; pa.qr = p.pqr;
   if ((rc = p.geo ? launch_prep_pixels_caps(pa, p.bcones, p.wcones, st) : launch_prep_pixels(pa, st))) return rc;

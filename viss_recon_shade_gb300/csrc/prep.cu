@@ -22,33 +22,53 @@ __device__ __forceinline__ float4 prep_pixel(const PixPrepArgs& a, int64_t pos) 
     return make_float4(0.f, 0.f, 0.f, 0.f);
   }
   const int64_t j = a.perm ? (int64_t)a.perm[pos] : pos;
-  const double x = a.sl * (double)a.l[j];
-  const double y = a.sm * (double)a.m[j];
-  const double z = a.sn * ((double)a.n[j] + a.n_offset);
   float b = 0.f;
   if (a.bright) {
     b = a.bright[j];
     if (a.trunc) b = (float)(int)b;  // int addFF = FF[..] (vissGen10M_shade.cu:128)
   }
-  const uint32_t A = fix32(x), B = fix32(y), C = fix32(z);
-  a.rec0[pos] = make_int4((int)A, (int)B, (int)C, __float_as_int(b));
-  if (a.rec1) {
+  const float lj = a.l[j], mj = a.m[j], nj = a.n[j];
+  uint32_t A, B, C;
+  float4 rec1, lo = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (a.pow2) {
+    // s is a power of two and s * n_offset * 2^32 an integer (s = 1 or 1/2, n_offset = -1 or 0):
+    // the products are exact in FP32 and the offset adds whole units after the rounding, so these are
+    // the double path's records without its ~15 FP64 operations a pixel
+    const float s32 = (float)(a.sl * 4294967296.0), s1 = (float)a.sl;
+    const float xa = lj * s32, ya = mj * s32, za = nj * s32;
+    A = (uint32_t)(unsigned long long)__float2ll_rn(xa);
+    B = (uint32_t)(unsigned long long)__float2ll_rn(ya);
+    C = (uint32_t)(unsigned long long)__float2ll_rn(za) + (uint32_t)(unsigned long long)a.off32;
+    rec1 = make_float4(lj * s1, mj * s1, nj * s1, __int_as_float((int)j));
+    if (a.lo)
+      lo = make_float4((xa - rintf(xa)) * 0x1p-32f, (ya - rintf(ya)) * 0x1p-32f, (za - rintf(za)) * 0x1p-32f, 0.f);
+  } else {
+    const double x = a.sl * (double)lj;
+    const double y = a.sm * (double)mj;
+    const double z = a.sn * ((double)nj + a.n_offset);
+    A = fix32(x);
+    B = fix32(y);
+    C = fix32(z);
     // coordinates for the fractional part of uvw; z without the n_offset shift (|s*n| <= 1)
-    a.rec1[pos] = make_int4(__float_as_int((float)x), __float_as_int((float)y),
-                            __float_as_int((float)(a.sn * (double)a.n[j])), (int)j);
+    rec1 = make_float4((float)x, (float)y, (float)(a.sn * (double)nj), __int_as_float((int)j));
+    if (a.lo) {
+      const double sc = 4294967296.0;
+      const double xa = x * sc, ya = y * sc, za = z * sc;
+      lo = make_float4((float)((xa - rint(xa)) / sc), (float)((ya - rint(ya)) / sc), (float)((za - rint(za)) / sc), 0.f);
+    }
   }
-  if (a.lo) {
-    const double sc = 4294967296.0;
-    const double xa = x * sc, ya = y * sc, za = z * sc;
-    a.lo[pos] = make_float4((float)((xa - rint(xa)) / sc), (float)((ya - rint(ya)) / sc),
-                          (float)((za - rint(za)) / sc), 0.f);
-  }
+  a.rec0[pos] = make_int4((int)A, (int)B, (int)C, __float_as_int(b));
+  if (a.rec1) reinterpret_cast<float4*>(a.rec1)[pos] = rec1;
+  if (a.lo) a.lo[pos] = lo;
   float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
   if (a.geo) {
-    const double gx = a.l[j], gy = a.m[j], gz = a.n[j];
-    const double nn = gx * gx + gy * gy + gz * gz;
-    const double inv = nn > 0 ? rsqrt(nn) : 0.0;
-    g = make_float4((float)(gx * inv), (float)(gy * inv), (float)(gz * inv), __int_as_float((int)j));
+    // unit direction, scaled by the largest coordinate first (good to 2e-7, against the 2e-6 of
+    // the limb within which the test is re-decided from the inputs)
+    const float big = fmaxf(fabsf(lj), fmaxf(fabsf(mj), fabsf(nj)));
+    const float gx = lj / big, gy = mj / big, gz = nj / big;
+    const float inv = big > 0.f ? 1.0f / sqrtf(fmaf(gx, gx, fmaf(gy, gy, gz * gz))) : 0.f;
+    g = big > 0.f ? make_float4(gx * inv, gy * inv, gz * inv, 0.f) : make_float4(0.f, 0.f, 0.f, 0.f);
+    g.w = __int_as_float((int)j);
     a.geo[pos] = g;
   }
   if (a.qr) {
@@ -266,12 +286,19 @@ __global__ void prep_rows_kernel(RowPrepArgs a, bool recon) {
     if (a.win) a.win[pr] = recon ? make_int4(0, 0, 0, 0) : make_int4(1, 0, 0, 0);
     return;
   }
-  const double uu = a.u[k], vv = a.v[k], ww = a.w[k];
-  const double Uu = floor(uu + 0.5), Uv = floor(vv + 0.5), Uw = floor(ww + 0.5);
-  const double lim = 1073741824.0;  // |U| < 2^30
-  if (!(fabs(Uu) < lim && fabs(Uv) < lim && fabs(Uw) < lim)) atomicOr(a.flags + FLAG_ERR, 1);
-  const double fu = uu - Uu, fv = vv - Uv, fw = ww - Uw;  // exact, in [-1/2, 1/2)
-  if (fu != 0.0 || fv != 0.0 || fw != 0.0) atomicOr(a.flags + FLAG_FRAC, 1);
+  // u = U + f, U the nearest integer, |f| <= 1/2: exact in FP32 (f has no bit below u's last)
+  const float u3[3] = {a.u[k], a.v[k], a.w[k]};
+  float U3[3], f3[3];
+  bool ok = true, frac = false;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    U3[c] = rintf(u3[c]);
+    f3[c] = u3[c] - U3[c];
+    ok &= fabsf(U3[c]) < 1073741824.f;  // |U| < 2^30; false for NaN
+    frac |= f3[c] != 0.f;
+  }
+  if (!ok) atomicOr(a.flags + FLAG_ERR, 1);
+  if (frac) atomicOr(a.flags + FLAG_FRAC, 1);
   if (a.rowsat) {
     int packed = PAD_PACKED;
     const int s = a.snap[k];
@@ -283,7 +310,7 @@ __global__ void prep_rows_kernel(RowPrepArgs a, bool recon) {
   }
   // PHASE_BIAS plus the per-row part of f_w * z: f_w * sn * n_offset; the
   // reconstruction folds the visibility's phase in too: y e^{ix} = |y| e^{i(x + arg y)}
-  uint32_t bias = (uint32_t)PHASE_BIAS + fix32(fw * a.sn * a.n_offset);
+  uint32_t bias = (uint32_t)PHASE_BIAS + (a.n_offset != 0.0 ? fix32((double)f3[2] * a.sn * a.n_offset) : 0u);
   float c = 0.f;
   if (recon) {
     const double wg = a.wgt ? (double)a.wgt[k] : 1.0;
@@ -298,10 +325,10 @@ __global__ void prep_rows_kernel(RowPrepArgs a, bool recon) {
       c = -c;
     }
   }
-  a.rows0[pr] = make_int4((int)(long long)Uu, (int)(long long)Uv, (int)(long long)Uw, (int)bias);
+  a.rows0[pr] = make_int4((int)(long long)U3[0], (int)(long long)U3[1], (int)(long long)U3[2], (int)bias);
   // the FP32 parts of the phase are summed in radians: coefficients times 2 pi
-  a.rows1[pr] = make_float4((float)(fu * (double)K2PI), (float)(fv * (double)K2PI), (float)(fw * (double)K2PI), c);
-  if (a.uf) a.uf[pr] = make_float4((float)(Uu * (double)K2PI), (float)(Uv * (double)K2PI), (float)(Uw * (double)K2PI), 0.f);
+  a.rows1[pr] = make_float4(f3[0] * K2PI, f3[1] * K2PI, f3[2] * K2PI, c);
+  if (a.uf) a.uf[pr] = make_float4(U3[0] * K2PI, U3[1] * K2PI, U3[2] * K2PI, 0.f);
   if (a.win) {
     int4 wv = recon ? make_int4(0, 0, 0, 0) : make_int4(1, 0, 0, 0);  // empty
     if (a.shade) {

@@ -105,7 +105,7 @@ enum PixClass : int { CLS_VIS = 0, CLS_OCC = 1, CLS_MIX = 2 };
 //   A  = round(x * 2^32) mod 2^32  -- the integer part of u multiplies it exactly mod 1 turn
 //   A' = round(x * 2^30)           -- for the fractional part of u (|x| < 2)
 //   lo = x - A*2^-32 (float)       -- compensation of the rounding of A
-// A visibility coordinate u is split u = U + f, U = floor(u + 1/2), f in [-1/2, 1/2).
+// A visibility coordinate u is split u = U + f, U the nearest integer, |f| <= 1/2.
 // Phase (turns * 2^32, mod 2^32) = U*A + V*B + W*C + bias_k; bias_k carries
 // PHASE_BIAS, f_w*s*n_offset and (reconstruction) the phase of the row's
 // visibility.  The fractional part delta = f_u*x + f_v*y + f_w*z' (FP32, z' = s*n,
@@ -209,6 +209,8 @@ struct PixPrepArgs {
   const float* bright;
   int64_t J, Jpad;
   double sl, sm, sn, n_offset;
+  int pow2;             // one scale, a power of two, and s * n_offset * 2^32 (off32) an integer
+  long long off32;
   int res;
   int trunc;
   int4* rec0;     // {A, B, C, bright bits}
