@@ -30,9 +30,6 @@ int device_sm_count() {
   return n;
 }
 
-int launch_prep_recon_ratios(const float* thetaP0, const float* phiP0, const float* dtheta, const float* dphi,
-                             int64_t K, int64_t Kpad, int4* win, int* flags, cudaStream_t st);
-
 static inline int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
 
 // ------------------------------------------------------------------ plans
@@ -362,6 +359,13 @@ static int check_ws(void* ws, size_t have, size_t need) {
 }
 
 // ------------------------------------------------------------------ passes
+static SatPrepArgs sat_args(const viss_geometry* geo, const viss_dft_cfg& cfg, float4* satdir, float4* cones) {
+  SatPrepArgs a{};
+  a.pos = geo->sat_pos; a.S = geo->S; a.nsat = geo->nsat; a.R = cfg.moon_radius_km;
+  a.satdir = satdir; a.cones = cones;
+  return a;
+}
+
 // The phase scales of a pixel prep, and whether its FP32 form is exact (PixPrepArgs::pow2).
 static void set_scales(PixPrepArgs& a, const double scale[3], double n_offset) {
   a.sl = scale[0]; a.sm = scale[1]; a.sn = scale[2]; a.n_offset = n_offset;
@@ -402,7 +406,8 @@ int vis_dft_impl(const viss_dft_cfg& cfg, const double scale[3], const float dlm
   VISS_CUDA(cudaMemsetAsync(p.flags, 0, FLAG_WORDS * sizeof(int), st));
   if (p.plain) {
     // the reference's form: one launch per channel
-    if (p.geo && (rc = launch_prep_satellites(geo->sat_pos, geo->S, geo->nsat, cfg.moon_radius_km, p.satdir, nullptr, st))) return rc;
+    if (p.geo && (rc = launch_prep(PixPrepArgs{}, RowPrepArgs{}, sat_args(geo, cfg, p.satdir, nullptr), false, st)))
+      return rc;
     for (int c = 0; c < bt.ch.nch; ++c) {
       const int64_t r0 = bt.ch.row_off[c], r1 = bt.ch.row_off[c + 1];
       if (r1 == r0) continue;
@@ -425,7 +430,6 @@ int vis_dft_impl(const viss_dft_cfg& cfg, const double scale[3], const float dlm
   pa.res = cfg.res; pa.trunc = map ? 0 : cfg.trunc_brightness;  // the map's base brightness is truncated per member
   pa.rec0 = p.pix0; pa.rec1 = p.pix1; pa.lo = p.plo; pa.geo = p.pgeo; pa.qr = p.pqr;
   pa.widx = p.ref ? widx : nullptr;
-  if ((rc = launch_prep_pixels(pa, st))) return rc;
   if (p.rrng && (rc = launch_prep_ref_ranges(widx, sky.J, p.Jpad / VIS_P, p.rrng, st))) return rc;
   RowPrepArgs ra{};
   ra.u = vis.u; ra.v = vis.v; ra.w = vis.w; ra.shade = vis.shade;
@@ -436,11 +440,8 @@ int vis_dft_impl(const viss_dft_cfg& cfg, const double scale[3], const float dlm
   ra.K = vis.K; ra.Kpad = p.Kpad; ra.mask_mode = cfg.mask_mode; ra.recon_mask = VISS_RECON_MASK_NONE;
   ra.rows0 = p.rows0; ra.rows1 = p.rows1; ra.rowsat = p.rowsat; ra.uf = p.rowsf; ra.win = p.win;
   ra.flags = p.flags;
-  if ((rc = launch_prep_rows(ra, false, st))) return rc;
-  if (p.geo) {
-    if ((rc = launch_prep_satellites(geo->sat_pos, geo->S, geo->nsat, cfg.moon_radius_km, p.satdir, nullptr, st))) return rc;
-    if ((rc = launch_prep_rowblock_cones(p.rowsat, p.satdir, bt.ch, p.nrb, p.cones, st))) return rc;
-  }
+  if ((rc = launch_prep(pa, ra, p.geo ? sat_args(geo, cfg, p.satdir, nullptr) : SatPrepArgs{}, false, st))) return rc;
+  if (p.geo && (rc = launch_prep_rowblock_cones(p.rowsat, p.satdir, bt.ch, p.nrb, p.cones, st))) return rc;
   VisParams vp{};
   vp.pix0 = p.pix0; vp.pix1 = p.pix1; vp.plo = p.plo; vp.pgeo = p.pgeo; vp.pqr = p.pqr;
   vp.rows0 = p.rows0; vp.rows1 = p.rows1; vp.rowsat = p.rowsat; vp.rowsf = p.rowsf; vp.win = p.win;
@@ -488,7 +489,8 @@ int recon_impl(const viss_dft_cfg& cfg, const double scale[3], const float dlmn[
       VISS_CUDA(cudaMemsetAsync(F2 + (int64_t)c * sky.J, 0, sizeof(float2) * (size_t)sky.J, st));
   if (p.plain) {
     // the reference's form: one launch per channel
-    if (p.geo && (rc = launch_prep_satellites(geo->sat_pos, geo->S, geo->nsat, cfg.moon_radius_km, p.satdir, nullptr, st))) return rc;
+    if (p.geo && (rc = launch_prep(PixPrepArgs{}, RowPrepArgs{}, sat_args(geo, cfg, p.satdir, nullptr), false, st)))
+      return rc;
     for (int c = 0; c < bt.ch.nch; ++c) {
       const int64_t r0 = bt.ch.row_off[c], r1 = bt.ch.row_off[c + 1];
       if (r1 == r0) continue;
@@ -525,7 +527,7 @@ int recon_impl(const viss_dft_cfg& cfg, const double scale[3], const float dlmn[
   set_scales(pa, scale, cfg.n_offset);
   pa.res = cfg.res; pa.trunc = 0;
   pa.rec0 = p.pix0; pa.rec1 = p.pix1; pa.lo = p.plo; pa.geo = p.pgeo; pa.qr = p.pqr;
-  if ((rc = p.geo ? launch_prep_pixels_caps(pa, p.bcones, p.wcones, st) : launch_prep_pixels(pa, st))) return rc;
+  pa.bcaps = p.bcones; pa.wcaps = p.wcones;
   RowPrepArgs ra{};
   ra.u = vis.u; ra.v = vis.v; ra.w = vis.w; ra.wgt = vis.wgt; ra.V = V;
   ra.shade = ratio_arrays ? nullptr : vis.shade;
@@ -536,16 +538,9 @@ int recon_impl(const viss_dft_cfg& cfg, const double scale[3], const float dlmn[
   ra.K = vis.K; ra.Kpad = p.Kpad; ra.mask_mode = VISS_MASK_NONE; ra.recon_mask = cfg.recon_mask;
   ra.rows0 = p.rows0; ra.rows1 = p.rows1; ra.rowsat = p.rowsat; ra.uf = p.rowsf; ra.win = p.win;
   ra.flags = p.flags;
-  if ((rc = launch_prep_rows(ra, true, st))) return rc;
-  if (p.ref && ratio_arrays) {
-    if ((rc = launch_prep_recon_ratios(ratio_arrays[0], ratio_arrays[1], ratio_arrays[2], ratio_arrays[3], vis.K,
-                                       p.Kpad, p.win, p.flags, st)))
-      return rc;
-  }
-  if (p.geo) {
-    if ((rc = launch_prep_satellites(geo->sat_pos, geo->S, geo->nsat, cfg.moon_radius_km, p.satdir, p.scones, st)))
-      return rc;
-  }
+  if (p.ref && ratio_arrays)
+    for (int i = 0; i < 4; ++i) ra.ratios[i] = ratio_arrays[i];
+  if ((rc = launch_prep(pa, ra, p.geo ? sat_args(geo, cfg, p.satdir, p.scones) : SatPrepArgs{}, true, st))) return rc;
   ReconParams rp{};
   rp.pix0 = p.pix0; rp.pix1 = p.pix1; rp.plo = p.plo; rp.pgeo = p.pgeo; rp.pqr = p.pqr;
   rp.rows0 = p.rows0; rp.rows1 = p.rows1; rp.rowsat = p.rowsat; rp.rowsf = p.rowsf; rp.win = p.win;

@@ -81,10 +81,8 @@ __device__ __forceinline__ float4 prep_pixel(const PixPrepArgs& a, int64_t pos) 
   return g;
 }
 
-__global__ void prep_pixels_kernel(const PixPrepArgs a) {
-  const int64_t pos = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (pos < a.Jpad) prep_pixel(a, pos);
-}
+constexpr int PREP_THREADS = 256;  // every part of prep_kernel
+static_assert(PREP_THREADS == REC_THREADS, "the caps' blocks are the recon's");
 
 __device__ __forceinline__ float warp_sum(float x) {
   for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
@@ -125,11 +123,11 @@ __device__ __forceinline__ void cap_write(const float4& axis, float c2, float4* 
 // The records and, on the way, the caps of each warp's patch of 32 * REC_TJ positions and of each
 // block of REC_PIX: one launch and no second read of the directions (two cap kernels with
 // FP64 cosines and arc cosines took 22 us beside 5 us of records on 2,048-12,288 pixels).
-__global__ void __launch_bounds__(REC_THREADS) prep_pixels_caps_kernel(const PixPrepArgs a, float4* bcaps, float4* wcaps) {
+__device__ void prep_pixels_caps(const PixPrepArgs& a, int block, float4* bcaps, float4* wcaps) {
   __shared__ float4 s_sum[REC_THREADS / 32];
   __shared__ float s_c2[REC_THREADS / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t p0 = (int64_t)blockIdx.x * REC_PIX + warp * 32 * REC_TJ + lane;
+  const int64_t p0 = (int64_t)block * REC_PIX + warp * 32 * REC_TJ + lane;
   float4 g[REC_TJ];
   float sx = 0.f, sy = 0.f, sz = 0.f;
 #pragma unroll
@@ -145,7 +143,7 @@ __global__ void __launch_bounds__(REC_THREADS) prep_pixels_caps_kernel(const Pix
     if (p0 + 32 * i < a.J) c2 = fmaxf(c2, chord2(wa, g[i]));
   c2 = warp_max(c2);
   if (lane == 0) {
-    cap_write(wa, c2, wcaps + 2 * ((int64_t)blockIdx.x * (REC_THREADS / 32) + warp));
+    cap_write(wa, c2, wcaps + 2 * ((int64_t)block * (REC_THREADS / 32) + warp));
     s_sum[warp] = make_float4(sx, sy, sz, 0.f);
   }
   __syncthreads();
@@ -163,15 +161,8 @@ __global__ void __launch_bounds__(REC_THREADS) prep_pixels_caps_kernel(const Pix
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int w = 1; w < REC_THREADS / 32; ++w) c2 = fmaxf(c2, s_c2[w]);
-    cap_write(ba, c2, bcaps + 2 * blockIdx.x);
+    cap_write(ba, c2, bcaps + 2 * (int64_t)block);
   }
-}
-
-int launch_prep_pixels_caps(const PixPrepArgs& a, float4* bcaps, float4* wcaps, cudaStream_t st) {
-  if (a.Jpad <= 0) return VISS_OK;
-  prep_pixels_caps_kernel<<<(unsigned)(a.Jpad / REC_PIX), REC_THREADS, 0, st>>>(a, bcaps, wcaps);
-  VISS_LAUNCH_CHECK("prep_pixels_caps_kernel");
-  return VISS_OK;
 }
 
 // {min, max} of widx over each run of VIS_P positions (the fine indices a vis
@@ -191,55 +182,6 @@ int launch_prep_ref_ranges(const int32_t* widx, int64_t J, int64_t ntiles, int2*
   if (ntiles <= 0) return VISS_OK;
   ref_ranges_kernel<<<(unsigned)((ntiles + 127) / 128), 128, 0, st>>>(widx, J, ntiles, rng);
   VISS_LAUNCH_CHECK("ref_ranges_kernel");
-  return VISS_OK;
-}
-
-// ------------------------------------------------------------- pixel order
-// Spatial order of the sky for the geometric mask: the direction is projected
-// on the face of the cube it points to and the face coordinates (10 bits each)
-// are interleaved (Morton), so consecutive positions are neighbouring pixels
-// and a warp's pixels see the Moon's limb together.
-// 10 bits -> the even bits of 20 (2-D Morton interleave)
-__device__ __forceinline__ uint32_t spread10(uint32_t x) {
-  x &= 0x3ff;
-  x = (x | (x << 8)) & 0x00ff00ffu;
-  x = (x | (x << 4)) & 0x0f0f0f0fu;
-  x = (x | (x << 2)) & 0x33333333u;
-  x = (x | (x << 1)) & 0x55555555u;
-  return x;
-}
-
-__global__ void pixel_keys_kernel(const float* l, const float* m, const float* n, int64_t J, uint32_t* keys,
-                                  int32_t* idx) {
-  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= J) return;
-  const float x = l[j], y = m[j], z = n[j];
-  const float ax = fabsf(x), ay = fabsf(y), az = fabsf(z);
-  uint32_t face;
-  float a, b, d;
-  if (ax >= ay && ax >= az) { face = x >= 0 ? 0 : 1; a = y; b = z; d = ax; }
-  else if (ay >= az) { face = y >= 0 ? 2 : 3; a = x; b = z; d = ay; }
-  else { face = z >= 0 ? 4 : 5; a = x; b = y; d = az; }
-  const float inv = d > 0.f ? 1.0f / d : 0.f;
-  const uint32_t ia = (uint32_t)fminf(1023.f, fmaxf(0.f, (a * inv + 1.0f) * 511.5f));
-  const uint32_t ib = (uint32_t)fminf(1023.f, fmaxf(0.f, (b * inv + 1.0f) * 511.5f));
-  keys[j] = (face << 20) | (spread10(ia) << 1) | spread10(ib);
-  idx[j] = (int32_t)j;
-}
-
-int launch_pixel_keys(const float* l, const float* m, const float* n, int64_t J, uint32_t* keys, int32_t* idx,
-                      cudaStream_t st) {
-  if (J <= 0) return VISS_OK;
-  pixel_keys_kernel<<<(unsigned)((J + 255) / 256), 256, 0, st>>>(l, m, n, J, keys, idx);
-  VISS_LAUNCH_CHECK("pixel_keys_kernel");
-  return VISS_OK;
-}
-
-int launch_prep_pixels(const PixPrepArgs& a, cudaStream_t st) {
-  if (a.Jpad <= 0) return VISS_OK;
-  const int bs = 256;
-  prep_pixels_kernel<<<(unsigned)((a.Jpad + bs - 1) / bs), bs, 0, st>>>(a);
-  VISS_LAUNCH_CHECK("prep_pixels_kernel");
   return VISS_OK;
 }
 
@@ -274,9 +216,7 @@ __device__ __forceinline__ int64_t padded_row_source(const ChannelRows& ch, int6
   return k < ch.row_off[lo + 1] ? k : -1;
 }
 
-__global__ void prep_rows_kernel(RowPrepArgs a, bool recon) {
-  const int64_t pr = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (pr >= a.Kpad) return;
+__device__ __forceinline__ void prep_row(const RowPrepArgs& a, bool recon, int64_t pr) {
   const int64_t k = a.padded ? padded_row_source(a.ch, pr) : (pr < a.K ? pr : -1);
   if (k < 0) {
     a.rows0[pr] = make_int4(0, 0, 0, PHASE_BIAS);
@@ -344,34 +284,18 @@ __global__ void prep_rows_kernel(RowPrepArgs a, bool recon) {
         const float r1 = (float)M1 / (float)M2, r2 = (float)M3 / (float)M4;
         wv = make_int4(recon_ratio_tmax(r1), recon_ratio_tmax(r2), 0, 0);
       }
+    } else if (a.ratios[0]) {
+      // viss_imagerecon gives the ratios themselves.  Skip iff fabsf(t0 - thetaP) < dt &&
+      // fabsf(p0 - phiP) < dp; the reference passes the same ratio array twice (t0 == dt,
+      // p0 == dp, :514-517); rows of another form set flag bit 4 and the call is rejected.
+      const float t0 = a.ratios[0][k], p0 = a.ratios[1][k], dt = a.ratios[2][k], dp = a.ratios[3][k];
+      const bool same_t = (t0 == dt) || (t0 != t0 && dt != dt);
+      const bool same_p = (p0 == dp) || (p0 != p0 && dp != dp);
+      if (!same_t || !same_p) atomicOr(a.flags + FLAG_ERR, 4);
+      wv = make_int4(recon_ratio_tmax(t0), recon_ratio_tmax(p0), 0, 0);
     }
     a.win[pr] = wv;
   }
-}
-
-int launch_prep_rows(const RowPrepArgs& a, bool recon, cudaStream_t st) {
-  if (a.Kpad <= 0) return VISS_OK;
-  const int bs = 256;
-  prep_rows_kernel<<<(unsigned)((a.Kpad + bs - 1) / bs), bs, 0, st>>>(a, recon);
-  VISS_LAUNCH_CHECK("prep_rows_kernel");
-  return VISS_OK;
-}
-
-// Reference recon ratio arrays given directly (viss_imagerecon): same tmax rule.
-__global__ void prep_recon_ratios_kernel(const float* thetaP0, const float* phiP0, const float* dtheta,
-                                         const float* dphi, int64_t K, int64_t Kpad, int4* win,
-                                         int* flags) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= Kpad) return;
-  if (k >= K) { win[k] = make_int4(0, 0, 0, 0); return; }
-  // skip iff fabsf(t0 - thetaP) < dt && fabsf(p0 - phiP) < dp.  The reference
-  // passes the same ratio array twice (t0 == dt, p0 == dp, :514-517); rows
-  // of another form set flag bit 4 and the call is rejected.
-  const float t0 = thetaP0[k], dt = dtheta[k], p0 = phiP0[k], dp = dphi[k];
-  const bool same_t = (t0 == dt) || (t0 != t0 && dt != dt);
-  const bool same_p = (p0 == dp) || (p0 != p0 && dp != dp);
-  if (!same_t || !same_p) atomicOr(flags + 1, 4);
-  win[k] = make_int4(recon_ratio_tmax(t0), recon_ratio_tmax(p0), 0, 0);
 }
 
 // ------------------------------------------------------------- satellites
@@ -426,15 +350,17 @@ __device__ __forceinline__ bool no_cone(const float4& d) { return d.w == 0.f; }
 // Satellite directions and (cones != NULL) each snapshot's cone: a thread per satellite, G
 // lanes (a power of two >= nsat) per snapshot, so that a pass of a hundred snapshots is a few
 // short chains (one thread per snapshot with FP64 arc cosines took 20 us, the directions 5.5).
-__global__ void prep_satellites_kernel(const float* pos, int64_t S, int nsat, int G, double R, float4* satdir,
-                                       float4* cones) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void prep_satellite(const SatPrepArgs& a, int64_t t) {
+  const int nsat = a.nsat, G = a.G;
+  const int64_t S = a.S;
+  float4* const satdir = a.satdir;
+  float4* const cones = a.cones;
   const int64_t s = t / G;
   const int i = (int)(t & (G - 1));
   const bool live = s < S && i < nsat;
   float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
   if (live) {
-    d = sat_direction(pos + 3 * (s * nsat + i), R);
+    d = sat_direction(a.pos + 3 * (s * nsat + i), a.R);
     satdir[s * nsat + i] = d;
   }
   if (!cones) return;
@@ -456,14 +382,45 @@ __global__ void prep_satellites_kernel(const float* pos, int64_t S, int nsat, in
   if (s < S && i == 0) cone_write(axis, c2, wmin, wmax, degen, cones + 2 * s);
 }
 
-int launch_prep_satellites(const float* sat_pos, int64_t S, int nsat, double R, float4* satdir, float4* cones,
-                           cudaStream_t st) {
-  if (S <= 0 || nsat <= 0) return VISS_OK;
-  int G = 1;
-  while (G < nsat) G <<= 1;
-  const int64_t n = S * G;
-  prep_satellites_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(sat_pos, S, nsat, G, R, satdir, cones);
-  VISS_LAUNCH_CHECK("prep_satellites_kernel");
+// The records of a pass in one launch: blocks of pixels, then of rows, then of satellites
+// (they do not depend on each other, and for a small pass each is a launch's latency
+// and little else: 3,360 x 2,048, vis and recon: 25 us in six launches, 10.5 in two).
+template <bool CAPS>
+__global__ void __launch_bounds__(PREP_THREADS) prep_kernel(const PixPrepArgs pix, const RowPrepArgs row, const SatPrepArgs sat,
+                                                            int pix_blocks, int row_blocks, bool recon) {
+  int b = (int)blockIdx.x;
+  if (b < pix_blocks) {
+    if (CAPS) prep_pixels_caps(pix, b, pix.bcaps, pix.wcaps);
+    else {
+      const int64_t pos = (int64_t)b * PREP_THREADS + threadIdx.x;
+      if (pos < pix.Jpad) prep_pixel(pix, pos);
+    }
+    return;
+  }
+  b -= pix_blocks;
+  if (b < row_blocks) {
+    const int64_t pr = (int64_t)b * PREP_THREADS + threadIdx.x;
+    if (pr < row.Kpad) prep_row(row, recon, pr);
+    return;
+  }
+  prep_satellite(sat, (int64_t)(b - row_blocks) * PREP_THREADS + threadIdx.x);
+}
+
+static int64_t prep_blocks(int64_t n) { return (n + PREP_THREADS - 1) / PREP_THREADS; }
+
+int launch_prep(const PixPrepArgs& pix, const RowPrepArgs& row, SatPrepArgs sat, bool recon, cudaStream_t st) {
+  const bool caps = pix.bcaps != nullptr;
+  const int64_t np = caps ? pix.Jpad / REC_PIX : prep_blocks(pix.Jpad), nr = prep_blocks(row.Kpad);
+  int64_t ns = 0;
+  if (sat.S > 0 && sat.nsat > 0) {
+    for (sat.G = 1; sat.G < sat.nsat;) sat.G <<= 1;
+    ns = prep_blocks(sat.S * sat.G);
+  }
+  const int64_t blocks = np + nr + ns;
+  if (blocks <= 0) return VISS_OK;
+  if (caps) prep_kernel<true><<<(unsigned)blocks, PREP_THREADS, 0, st>>>(pix, row, sat, (int)np, (int)nr, recon);
+  else prep_kernel<false><<<(unsigned)blocks, PREP_THREADS, 0, st>>>(pix, row, sat, (int)np, (int)nr, recon);
+  VISS_LAUNCH_CHECK("prep_kernel");
   return VISS_OK;
 }
 
@@ -547,15 +504,6 @@ int launch_prep_rowblock_cones(const int* rowsat, const float4* satdir, const Ch
   if (nblocks <= 0) return VISS_OK;
   rowblock_cones_kernel<<<(unsigned)nblocks, CONE_THREADS, 0, st>>>(rowsat, satdir, ch, cones);
   VISS_LAUNCH_CHECK("rowblock_cones_kernel");
-  return VISS_OK;
-}
-
-int launch_prep_recon_ratios(const float* thetaP0, const float* phiP0, const float* dtheta, const float* dphi,
-                             int64_t K, int64_t Kpad, int4* win, int* flags, cudaStream_t st) {
-  if (Kpad <= 0) return VISS_OK;
-  prep_recon_ratios_kernel<<<(unsigned)((Kpad + 255) / 256), 256, 0, st>>>(thetaP0, phiP0, dtheta, dphi, K,
-                                                                          Kpad, win, flags);
-  VISS_LAUNCH_CHECK("prep_recon_ratios_kernel");
   return VISS_OK;
 }
 

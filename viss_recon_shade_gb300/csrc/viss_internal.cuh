@@ -219,6 +219,18 @@ struct PixPrepArgs {
   float4* geo;    // {unit s, j bits}
   int2* qr;       // {i / res, i % res} of the fine index i the REF windows test
   const int32_t* widx;  // i = widx[j] (NULL: i = j)
+  float4* bcaps;        // recon, geometric: caps of the pixel blocks and of the warps' patches (or NULL)
+  float4* wcaps;
+};
+
+// Satellites of a geometric pass: directions and, for the reconstruction, snapshot cones.
+struct SatPrepArgs {
+  const float* pos;
+  int64_t S;
+  int nsat, G;      // G lanes per snapshot
+  double R;
+  float4* satdir;
+  float4* cones;    // or NULL
 };
 
 // Visibility rows of a (batched) pass: channel c owns input rows
@@ -246,6 +258,7 @@ struct RowPrepArgs {
   const float* wgt;
   const float* V;        // recon: K x 2, folded into bias and c
   const int32_t* shade;  // K x 4
+  const float* ratios[4];  // recon REF, in place of shade: thetaP0, phiP0, dtheta, dphi
   const int32_t* snap;
   const int32_t* pair;
   int nsat;
@@ -373,18 +386,12 @@ struct RecReduceParams {
 };
 
 // ------------------------------------------------------------- launchers
-int launch_prep_pixels(const PixPrepArgs& a, cudaStream_t st);
-int launch_pixel_keys(const float* l, const float* m, const float* n, int64_t J, uint32_t* keys, int32_t* idx,
-                      cudaStream_t st);
+int launch_prep(const PixPrepArgs& pix, const RowPrepArgs& row, SatPrepArgs sat, bool recon, cudaStream_t st);
 // Spatial permutation of the sky (keys, then a stable radix sort); scratch from
 // the caller's workspace.  perm[pos] = pixel.
 size_t pixel_order_scratch(int64_t J);
 int pixel_order(const float* l, const float* m, const float* n, int64_t J, void* scratch, size_t scratch_bytes,
                 int32_t* perm, cudaStream_t st);
-int launch_prep_rows(const RowPrepArgs& a, bool recon, cudaStream_t st);
-int launch_prep_pixels_caps(const PixPrepArgs& a, float4* bcaps, float4* wcaps, cudaStream_t st);
-int launch_prep_satellites(const float* sat_pos, int64_t S, int nsat, double R, float4* satdir, float4* cones,
-                           cudaStream_t st);
 int launch_prep_rowblock_cones(const int* rowsat, const float4* satdir, const ChannelRows& ch, int64_t nblocks,
                                float4* cones, cudaStream_t st);
 
