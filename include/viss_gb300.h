@@ -289,6 +289,23 @@ VISS_API int viss_imagerecon(int uvw_index, int lmnC_index, int res, float* F, c
                     const float* n, const float* uvwFrequencyMap, const float* thetaP0,
                     const float* phiP0, const float* dtheta, const float* dphi, float dl, float dm,
                     float dn, int precision, void* stream);
+/* The same on a caller workspace: with workspace NULL the size in bytes is stored in
+ * *workspace_bytes and nothing runs (a countLoc map is summed for it, which synchronises);
+ * otherwise *workspace_bytes is the size of the 256-byte aligned workspace.  A program that
+ * keeps one, or has an allocator that does, is spared cudaMallocAsync and cudaFreeAsync on
+ * each call, which map the memory anew after every synchronisation (~75 us a call). */
+VISS_API int viss_visscal_ws(int uvws_index, int lmnC_index, int res, const float* FF, float* viss,
+                 const float* u, const float* v, const float* w, const float* l, const float* m,
+                 const float* n, const int* shadeM1, const int* shadeM2, const int* shadeM3,
+                 const int* shadeM4, const float* NXq, const int* countLoc, float dl, float dm,
+                 float dn, int variant, int mask_mode, int precision, void* workspace,
+                 size_t* workspace_bytes, void* stream);
+VISS_API int viss_imagerecon_ws(int uvw_index, int lmnC_index, int res, float* F, const float* viss,
+                 const float* u, const float* v, const float* w, const float* l, const float* m,
+                 const float* n, const float* uvwFrequencyMap, const float* thetaP0,
+                 const float* phiP0, const float* dtheta, const float* dphi, float dl, float dm,
+                 float dn, int precision, void* workspace, size_t* workspace_bytes, void* stream);
+
 
 /* ---------------------------------------------------------- orbit + uvw */
 typedef struct viss_orbit_cfg {  /* MIncline_generate_uvw_float.cu:22-30, 184-190 */

@@ -110,6 +110,11 @@ _SIGS = {
                                C.c_float, C.c_float, C.c_float, C.c_int, C.c_int, C.c_int, _P]),
     "viss_imagerecon": (C.c_int, [C.c_int, C.c_int, C.c_int, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P,
                                   C.c_float, C.c_float, C.c_float, C.c_int, _P]),
+    "viss_visscal_ws": (C.c_int, [C.c_int, C.c_int, C.c_int, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P,
+                                  C.c_float, C.c_float, C.c_float, C.c_int, C.c_int, C.c_int, _P, C.POINTER(C.c_size_t),
+                                  _P]),
+    "viss_imagerecon_ws": (C.c_int, [C.c_int, C.c_int, C.c_int, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P,
+                                     C.c_float, C.c_float, C.c_float, C.c_int, _P, C.POINTER(C.c_size_t), _P]),
     "viss_orbit_snapshots": (C.c_int64, [C.POINTER(OrbitCfg)]),
     "viss_orbit_positions": (C.c_int, [C.POINTER(OrbitCfg), _P, _P, _P]),
     "viss_baseline_uvw": (C.c_int, [_P, _P, C.c_int64, C.c_int32, C.c_int, C.c_double, C.c_int, _P, _P, _P, _P, _P,

@@ -101,7 +101,8 @@ def _positions(pos: torch.Tensor, dtype=torch.float32, name: str = "pos") -> tor
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # torch.cuda.current_stream().cuda_stream without building the Stream object (3 us a call)
+    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def _workspace(nbytes: int, device) -> Optional[torch.Tensor]:
@@ -402,6 +403,17 @@ def autotune_report(batch: ChannelBatch):
 
 
 # ---------------------------------------------------------------- reference-shaped
+def _on_workspace(fn, call, device, where: str) -> None:
+    """A reference-shaped entry point on a workspace of torch's allocator, which keeps it for the
+    next call (the plain entry points allocate and free with every call)."""
+    nb = C.c_size_t(0)
+    st = _stream()
+    L.check(fn(*call, None, C.byref(nb), st), where)
+    ws = _workspace(nb.value, device)
+    if ws is not None:
+        L.check(fn(*call, _ptr(ws), C.byref(nb), st), where)
+
+
 def visscal(uvws_index: int, lmnC_index: int, res: int, FF, viss, u, v, w, l, m, n, shadeM1, shadeM2, shadeM3,
             shadeM4, NXq=None, countLoc=None, dl: float = 2.0, dm: float = 2.0, dn: float = 2.0,
             variant: int = VARIANT_OPTIM, mask: int = MASK_REF_QUIRK, precision: int = PREC_FAST):
@@ -417,9 +429,12 @@ def visscal(uvws_index: int, lmnC_index: int, res: int, FF, viss, u, v, w, l, m,
     uu = [_dev(x, torch.float32, nm, K) for x, nm in ((u, "u"), (v, "v"), (w, "w"))]
     pix = [_dev(x, torch.float32, nm, J) for x, nm in ((l, "l"), (m, "m"), (n, "n"))]
     sh = [_dev(x, torch.int32, f"shadeM{i + 1}", K) for i, x in enumerate((shadeM1, shadeM2, shadeM3, shadeM4))]
-    L.check(L.lib.viss_visscal(K, J, int(res), _ptr(args[0]), _ptr(viss), *map(_ptr, uu), *map(_ptr, pix),
-                               *map(_ptr, sh), _ptr(NXq), _ptr(countLoc), float(dl), float(dm), float(dn),
-                               int(variant), int(mask), int(precision), _stream()), "viss_visscal")
+    call = (K, J, int(res), _ptr(args[0]), _ptr(viss), *map(_ptr, uu), *map(_ptr, pix), *map(_ptr, sh), _ptr(NXq),
+            _ptr(countLoc), float(dl), float(dm), float(dn), int(variant), int(mask), int(precision))
+    if countLoc is None:
+        _on_workspace(L.lib.viss_visscal_ws, call, viss.device, "viss_visscal")
+    else:  # the map's size is read back by the call: once, with its own workspace
+        L.check(L.lib.viss_visscal(*call, _stream()), "viss_visscal")
     return viss
 
 
@@ -436,9 +451,9 @@ def imagerecon(uvw_index: int, lmnC_index: int, res: int, F, viss, u, v, w, l, m
     wg = _dev(uvwFrequencyMap, torch.float32, "uvwFrequencyMap", K)
     rat = [_dev(x, torch.float32, nm, K) for x, nm in ((thetaP0, "thetaP0"), (phiP0, "phiP0"), (dtheta, "dtheta"),
                                                       (dphi, "dphi"))]
-    L.check(L.lib.viss_imagerecon(K, J, int(res), _ptr(F), _ptr(viss), *map(_ptr, uu), *map(_ptr, pix), _ptr(wg),
-                                  *map(_ptr, rat), float(dl), float(dm), float(dn), int(precision), _stream()),
-            "viss_imagerecon")
+    call = (K, J, int(res), _ptr(F), _ptr(viss), *map(_ptr, uu), *map(_ptr, pix), _ptr(wg), *map(_ptr, rat), float(dl),
+            float(dm), float(dn), int(precision))
+    _on_workspace(L.lib.viss_imagerecon_ws, call, F.device, "viss_imagerecon")
     return F
 
 

@@ -389,7 +389,7 @@ static viss_vis_set channel_rows(const viss_vis_set& vis, int64_t r0, int64_t r1
 int vis_dft_impl(const viss_dft_cfg& cfg, const double scale[3], const float dlmn[3], const viss_sky& sky,
                  const viss_vis_set& vis, const Batch& bt, const viss_geometry* geo, const Tuning& tn, float* V,
                  void* ws, size_t ws_bytes, cudaStream_t st, const viss_fine_map* map = nullptr,
-                 const int32_t* widx = nullptr) {
+                 const int32_t* widx = nullptr, const int* const* shade_cols = nullptr) {
   VisPlan p;
   plan_vis(p, cfg, bt, sky.J, geo, tn, map, widx != nullptr);
   // work items are counted in int (a caller's vis_split can ask for more)
@@ -433,6 +433,7 @@ int vis_dft_impl(const viss_dft_cfg& cfg, const double scale[3], const float dlm
   if (p.rrng && (rc = launch_prep_ref_ranges(widx, sky.J, p.Jpad / VIS_P, p.rrng, st))) return rc;
   RowPrepArgs ra{};
   ra.u = vis.u; ra.v = vis.v; ra.w = vis.w; ra.shade = vis.shade;
+  for (int i = 0; i < 4; ++i) ra.shade_cols[i] = shade_cols ? shade_cols[i] : nullptr;
   ra.snap = p.geo ? vis.snap : nullptr; ra.pair = p.geo ? vis.pair : nullptr;
   ra.nsat = geo ? geo->nsat : 0; ra.S = geo ? geo->S : 0;
   ra.sn = scale[2]; ra.n_offset = cfg.n_offset;
@@ -828,10 +829,11 @@ int viss_recon_batch(const viss_dft_cfg* cfg, const viss_sky* sky, const viss_vi
                     static_cast<cudaStream_t>(stream), nullptr);
 }
 
-int viss_visscal(int uvws_index, int lmnC_index, int res, const float* FF, float* viss, const float* u,
+static int visscal_impl(int uvws_index, int lmnC_index, int res, const float* FF, float* viss, const float* u,
                  const float* v, const float* w, const float* l, const float* m, const float* n, const int* shadeM1,
                  const int* shadeM2, const int* shadeM3, const int* shadeM4, const float* NXq, const int* countLoc,
-                 float dl, float dm, float dn, int variant, int mask_mode, int precision, void* stream) {
+                 float dl, float dm, float dn, int variant, int mask_mode, int precision, void* ws, size_t ws_bytes,
+                        size_t* query, void* stream) {
   if (uvws_index < 0 || lmnC_index < 0) return fail(VISS_ERR_RANGE, "negative size");
   if (!NXq != !countLoc) return fail(VISS_ERR_INVALID, "NXq and countLoc go together (both NULL: identity map)");
   if (!(dl > 0.f && dm > 0.f && dn > 0.f)) return fail(VISS_ERR_RANGE, "dl, dm, dn must be > 0");
@@ -858,6 +860,7 @@ int viss_visscal(int uvws_index, int lmnC_index, int res, const float* FF, float
   const double scale[3] = {1.0 / dl, 1.0 / dm, 1.0 / dn};
   const float dlmn[3] = {dl, dm, dn};
   viss_fine_map map{FF, NXq, nullptr, countLoc, 0};
+  const int* const cols[4] = {shadeM1, shadeM2, shadeM3, shadeM4};
   if (countLoc) {
     // the fine pixel count is not among the reference's arguments: sum(countLoc)
     if ((rc = sum_counts(countLoc, lmnC_index, &map.X, st))) return rc;
@@ -867,11 +870,15 @@ int viss_visscal(int uvws_index, int lmnC_index, int res, const float* FF, float
   if ((rc = make_batch(nullptr, uvws_index, cfg, bt))) return rc;
   VisPlan p;
   plan_vis(p, cfg, bt, lmnC_index, nullptr, Tuning{}, countLoc ? &map : nullptr);
-  const size_t shade_bytes = mask_mode != VISS_MASK_NONE ? ((sizeof(int4) * (size_t)uvws_index + 255) & ~size_t(255)) : 0;
-  void* ws = nullptr;
+  // the plain kernel reads packed windows, the row records take the four columns
+  const bool pack = mask_mode != VISS_MASK_NONE && plain_precision(precision);
+  const size_t shade_bytes = pack ? ((sizeof(int4) * (size_t)uvws_index + 255) & ~size_t(255)) : 0;
   const size_t total = p.bytes + shade_bytes;
-  if (total) VISS_CUDA(cudaMallocAsync(&ws, total, st));
-  if (shade_bytes && uvws_index > 0) {
+  if (query) { *query = total; return VISS_OK; }
+  if (ws && (rc = check_ws(ws, ws_bytes, total))) return rc;
+  const bool alloc = !ws && total > 0;
+  if (alloc) VISS_CUDA(cudaMallocAsync(&ws, total, st));
+  if (pack && uvws_index > 0) {
     int4* packed = reinterpret_cast<int4*>(static_cast<char*>(ws) + p.bytes);
     pack_shade_kernel<<<(unsigned)((uvws_index + 255) / 256), 256, 0, st>>>(shadeM1, shadeM2, shadeM3, shadeM4,
                                                                             uvws_index, packed);
@@ -879,18 +886,38 @@ int viss_visscal(int uvws_index, int lmnC_index, int res, const float* FF, float
     vis.shade = reinterpret_cast<const int32_t*>(packed);
   }
   rc = vis_dft_impl(cfg, scale, dlmn, sky, vis, bt, nullptr, Tuning{}, viss, ws, p.bytes, st,
-                    countLoc ? &map : nullptr);
-  if (ws) {
+                    countLoc ? &map : nullptr, nullptr, mask_mode != VISS_MASK_NONE && !pack ? cols : nullptr);
+  if (alloc) {
     cudaError_t e = cudaFreeAsync(ws, st);
     if (rc == VISS_OK && e != cudaSuccess) rc = cuda_fail(e, "cudaFreeAsync");
   }
   return rc;
 }
 
-int viss_imagerecon(int uvw_index, int lmnC_index, int res, float* F, const float* viss, const float* u,
+int viss_visscal(int uvws_index, int lmnC_index, int res, const float* FF, float* viss, const float* u,
+                 const float* v, const float* w, const float* l, const float* m, const float* n, const int* shadeM1,
+                 const int* shadeM2, const int* shadeM3, const int* shadeM4, const float* NXq, const int* countLoc,
+                 float dl, float dm, float dn, int variant, int mask_mode, int precision, void* stream) {
+  return visscal_impl(uvws_index, lmnC_index, res, FF, viss, u, v, w, l, m, n, shadeM1, shadeM2, shadeM3, shadeM4, NXq,
+                      countLoc, dl, dm, dn, variant, mask_mode, precision, nullptr, 0, nullptr, stream);
+}
+
+int viss_visscal_ws(int uvws_index, int lmnC_index, int res, const float* FF, float* viss, const float* u,
+                 const float* v, const float* w, const float* l, const float* m, const float* n, const int* shadeM1,
+                 const int* shadeM2, const int* shadeM3, const int* shadeM4, const float* NXq, const int* countLoc,
+                 float dl, float dm, float dn, int variant, int mask_mode, int precision, void* workspace, size_t* workspace_bytes,
+                    void* stream) {
+  if (!workspace_bytes) return fail(VISS_ERR_INVALID, "workspace_bytes is NULL");
+  return visscal_impl(uvws_index, lmnC_index, res, FF, viss, u, v, w, l, m, n, shadeM1, shadeM2, shadeM3, shadeM4, NXq,
+                      countLoc, dl, dm, dn, variant, mask_mode, precision, workspace, *workspace_bytes,
+                      workspace ? nullptr : workspace_bytes, stream);
+}
+
+static int imagerecon_impl(int uvw_index, int lmnC_index, int res, float* F, const float* viss, const float* u,
                     const float* v, const float* w, const float* l, const float* m, const float* n,
                     const float* uvwFrequencyMap, const float* thetaP0, const float* phiP0, const float* dtheta,
-                    const float* dphi, float dl, float dm, float dn, int precision, void* stream) {
+                    const float* dphi, float dl, float dm, float dn, int precision, void* ws, size_t ws_bytes, size_t* query,
+                           void* stream) {
   if (uvw_index < 0 || lmnC_index < 0) return fail(VISS_ERR_RANGE, "negative size");
   if (!(dl > 0.f && dm > 0.f && dn > 0.f)) return fail(VISS_ERR_RANGE, "dl, dm, dn must be > 0");
   const bool masked = thetaP0 && phiP0 && dtheta && dphi;
@@ -916,8 +943,10 @@ int viss_imagerecon(int uvw_index, int lmnC_index, int res, float* F, const floa
   if ((rc = make_batch(nullptr, uvw_index, cfg, bt))) return rc;
   RecPlan p;
   plan_recon(p, cfg, bt, lmnC_index, nullptr, Tuning{});
-  void* ws = nullptr;
-  if (p.bytes) VISS_CUDA(cudaMallocAsync(&ws, p.bytes, st));
+  if (query) { *query = p.bytes; return VISS_OK; }
+  if (ws && (rc = check_ws(ws, ws_bytes, p.bytes))) return rc;
+  const bool alloc = !ws && p.bytes > 0;
+  if (alloc) VISS_CUDA(cudaMallocAsync(&ws, p.bytes, st));
   const float* ratios[4] = {thetaP0, phiP0, dtheta, dphi};
   rc = recon_impl(cfg, scale, dlmn, sky, vis, bt, nullptr, Tuning{}, viss, F, ws, p.bytes, st,
                   masked ? ratios : nullptr);
@@ -930,11 +959,29 @@ int viss_imagerecon(int uvw_index, int lmnC_index, int res, float* F, const floa
     if (e != cudaSuccess) rc = cuda_fail(e, "flag readback");
     else if (flags[FLAG_ERR] & 4) rc = fail(VISS_ERR_UNSUPPORTED, "thetaP0 != dtheta or phiP0 != dphi");
   }
-  if (ws) {
+  if (alloc) {
     cudaError_t e = cudaFreeAsync(ws, st);
     if (rc == VISS_OK && e != cudaSuccess) rc = cuda_fail(e, "cudaFreeAsync");
   }
   return rc;
+}
+
+int viss_imagerecon(int uvw_index, int lmnC_index, int res, float* F, const float* viss, const float* u,
+                    const float* v, const float* w, const float* l, const float* m, const float* n,
+                    const float* uvwFrequencyMap, const float* thetaP0, const float* phiP0, const float* dtheta,
+                    const float* dphi, float dl, float dm, float dn, int precision, void* stream) {
+  return imagerecon_impl(uvw_index, lmnC_index, res, F, viss, u, v, w, l, m, n, uvwFrequencyMap, thetaP0, phiP0, dtheta, dphi,
+                         dl, dm, dn, precision, nullptr, 0, nullptr, stream);
+}
+
+int viss_imagerecon_ws(int uvw_index, int lmnC_index, int res, float* F, const float* viss, const float* u,
+                    const float* v, const float* w, const float* l, const float* m, const float* n,
+                    const float* uvwFrequencyMap, const float* thetaP0, const float* phiP0, const float* dtheta,
+                    const float* dphi, float dl, float dm, float dn, int precision, void* workspace, size_t* workspace_bytes,
+                       void* stream) {
+  if (!workspace_bytes) return fail(VISS_ERR_INVALID, "workspace_bytes is NULL");
+  return imagerecon_impl(uvw_index, lmnC_index, res, F, viss, u, v, w, l, m, n, uvwFrequencyMap, thetaP0, phiP0, dtheta, dphi,
+                         dl, dm, dn, precision, workspace, *workspace_bytes, workspace ? nullptr : workspace_bytes, stream);
 }
 
 }  // extern "C"

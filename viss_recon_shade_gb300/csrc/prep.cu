@@ -271,9 +271,10 @@ __device__ __forceinline__ void prep_row(const RowPrepArgs& a, bool recon, int64
   if (a.uf) a.uf[pr] = make_float4(U3[0] * K2PI, U3[1] * K2PI, U3[2] * K2PI, 0.f);
   if (a.win) {
     int4 wv = recon ? make_int4(0, 0, 0, 0) : make_int4(1, 0, 0, 0);  // empty
-    if (a.shade) {
-      const int M1 = a.shade[4 * k], M2 = a.shade[4 * k + 1], M3 = a.shade[4 * k + 2],
-                M4 = a.shade[4 * k + 3];
+    if (a.shade || a.shade_cols[0]) {
+      const int M1 = a.shade ? a.shade[4 * k] : a.shade_cols[0][k], M2 = a.shade ? a.shade[4 * k + 1] : a.shade_cols[1][k],
+                M3 = a.shade ? a.shade[4 * k + 2] : a.shade_cols[2][k],
+                M4 = a.shade ? a.shade[4 * k + 3] : a.shade_cols[3][k];
       if (!recon) {
         if (a.mask_mode == VISS_MASK_REF_QUIRK) {
           if (M3 <= 0 && M4 >= 0) wv = make_int4(0, M4, M1, M2);

@@ -258,6 +258,7 @@ struct RowPrepArgs {
   const float* wgt;
   const float* V;        // recon: K x 2, folded into bias and c
   const int32_t* shade;  // K x 4
+  const int* shade_cols[4];  // vis REF: the four columns instead
   const float* ratios[4];  // recon REF, in place of shade: thetaP0, phiP0, dtheta, dphi
   const int32_t* snap;
   const int32_t* pair;
