@@ -17,7 +17,7 @@
 set -euo pipefail
 REF="${1:-${VISS_REFERENCE_DIR:-/root/reference}}"
 OUT="$(cd "$(dirname "$0")" && pwd)/_ref"
-[ -d "$REF" ] || { echo "reference sources not present: $REF" >&2; exit 0; }
+compgen -G "$REF/*.cu" > /dev/null || { echo "reference sources not present: $REF" >&2; exit 0; }
 mkdir -p "$OUT"
 rm -f "$OUT"/*.ptx
 FILES="vissGen10M_shade vissGen10M_shade_optim1 vissGen10M_shade_optim2 vissGen1M_shade_optim1 \
