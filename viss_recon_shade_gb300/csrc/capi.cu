@@ -240,13 +240,12 @@ struct RecPlan {
 // Recon work: every channel's rows cut into segments of about L rows, L chosen
 // for ~rec_items work items (segment x pixel block) per resident CTA; at most
 // VISS_MAX_SEG segments.  Segments are ordered longest first.
-static void plan_segments(RecPlan& p, const Batch& bt, const Tuning& tn) {
+static void plan_segments(RecPlan& p, const viss_dft_cfg& cfg, const Batch& bt, const Tuning& tn) {
   int64_t unit = REC_Q;
   const int nch = bt.ch.nch;
   // items per CTA: many short segments balance blocks whose pixels the Moon hides for
   // different parts of the orbit (10 MHz recon: 4 items 191 ms, 8 176 ms, 32 167 ms, 64 165 ms)
-  // resident CTAs: VISS_REC_MINB for the geometric kernel, one more for the others (recon.cu)
-  const int64_t target = (tn.rec_items > 0 ? tn.rec_items : 64) * planned_ctas(tn, p.geo ? VISS_REC_MINB : VISS_REC_MINB + 1);
+  const int64_t target = (tn.rec_items > 0 ? tn.rec_items : 64) * planned_ctas(tn, rec_ctas(cfg.recon_mask, p.comp));
   int64_t L = p.npb > 0 ? (p.K * p.npb + target - 1) / target : p.K;
   // A small pass has fewer than 4 segments of REC_Q rows per CTA: shorter ones, down to
   // REC_MIN_ROWS, so that every SM has work.  3,360 rows x 2,048 pixels: 58 -> 20 us;
@@ -305,7 +304,7 @@ static void plan_recon(RecPlan& p, const viss_dft_cfg& cfg, const Batch& bt, int
   p.npb = p.Jpad / REC_PIX;
   p.S = (geo && p.geo) ? geo->S : 0;
   p.nsd = (geo && p.geo) ? geo->S * (int64_t)geo->nsat : 0;
-  if (!p.plain) plan_segments(p, bt, tn);
+  if (!p.plain) plan_segments(p, cfg, bt, tn);
   p.layout(nullptr);
 }
 

@@ -25,6 +25,8 @@
 // Persistent CTAs take items from an atomic counter, longest segments first.
 // A channel split into several segments leaves partial sums per segment,
 // reduced in a fixed order.
+#include <type_traits>
+
 #include "viss_internal.cuh"
 
 namespace viss {
@@ -51,29 +53,275 @@ __device__ __forceinline__ void rec_term(const int4& r0, const float4& r1, const
   fi = fmaf(c, sn, fi);
 }
 
-constexpr int RM_NONE = 0, RM_REF = 1, RM_GEO = 2;
+// Two FP32 values in one 64-bit register pair; sm_103a's packed operations round each half as
+// the single ones do.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+
+// sin and cos of two angles (half a turn added), weighted into packed sums.
+__device__ __forceinline__ void sincos2(f32x2 x, f32x2 c, f32x2& fr, f32x2& fi) {
+  float xa, xb, sa, ca, sb, cb;
+  unpack2(x, xa, xb);
+  __sincosf(xa, &sa, &ca);
+  __sincosf(xb, &sb, &cb);
+  fr = fma2(c, pack2(ca, cb), fr);
+  fi = fma2(c, pack2(sa, sb), fi);
+}
+
+// Two terms without the SFU, for phases that are all fixed point (integer uvw): the top bit of
+// the phase (shifted by a quarter turn) is the sign of the term, the next 23 bits the
+// angle r in half turns, |r| <= 1/2, and sin(pi r) and cos(pi r) are polynomials in r^2 (least
+// maximum error by iteratively reweighted least squares; in FP32 they are off by 6e-8 rms,
+// the SFU's values with their angle by 2.6e-7).
+constexpr uint32_t POLY_BIAS = 128u + 0xC0000000u - (uint32_t)PHASE_BIAS;  // on top of the phase bias
+__device__ __forceinline__ void poly2(uint32_t qa, uint32_t qb, f32x2 c, f32x2& fr, f32x2& fi) {
+  qa += POLY_BIAS;
+  qb += POLY_BIAS;
+  // bit 23 of q >> 8 falls on a bit that is set in 1.0f
+  const f32x2 r = add2(pack2(__uint_as_float((qa >> 8) | 0x3f800000u), __uint_as_float((qb >> 8) | 0x3f800000u)),
+                       pack2(-1.5f, -1.5f));
+  float ca, cb;
+  unpack2(c, ca, cb);
+  const f32x2 cs = pack2(__uint_as_float(__float_as_uint(ca) ^ (qa & 0x80000000u)),
+                         __uint_as_float(__float_as_uint(cb) ^ (qb & 0x80000000u)));
+  const f32x2 y = mul2(r, r);
+  f32x2 s = fma2(y, pack2(0.0772222504f, 0.0772222504f), pack2(-0.598046422f, -0.598046422f));
+  f32x2 k = fma2(y, pack2(0.219696805f, 0.219696805f), pack2(-1.33188021f, -1.33188021f));
+  s = fma2(y, s, pack2(2.55003166f, 2.55003166f));
+  k = fma2(y, k, pack2(4.05841208f, 4.05841208f));
+  s = fma2(y, s, pack2(-5.16770697f, -5.16770697f));
+  k = fma2(y, k, pack2(-4.934793f, -4.934793f));
+  s = fma2(y, s, pack2(3.1415925f, 3.1415925f));
+  k = fma2(y, k, pack2(0.99999994f, 0.99999994f));
+  fr = fma2(cs, k, fr);
+  fi = fma2(cs, mul2(r, s), fi);
+}
+
+// One visibility row's terms with two of the thread's pixels.  The row's FP32 parts stand
+// twice in shared memory ({fu, fu, fv, fv}, {fw, fw, c, c}) as packed operands.  POLY: without
+// the SFU (integer uvw only).
+template <bool FRAC, bool COMP, bool POLY>
+__device__ __forceinline__ void rec_term2(const int4& r0, const ulonglong2& fuv, f32x2 fw, const float4& rf, f32x2 c,
+                                          const int* A, const int* B, const int* C, f32x2 X, f32x2 Y, f32x2 Z, f32x2 lx,
+                                          f32x2 ly, f32x2 lz, f32x2& fr, f32x2& fi) {
+  uint32_t q[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    q[h] = (uint32_t)r0.x * (uint32_t)A[h] + (uint32_t)r0.y * (uint32_t)B[h] + (uint32_t)r0.z * (uint32_t)C[h] +
+           (uint32_t)r0.w;
+  if (POLY) {
+    poly2(q[0], q[1], c, fr, fi);
+    return;
+  }
+  f32x2 e = pack2(KM3PI, KM3PI);
+  if (FRAC) e = fma2(fuv.x, X, fma2(fuv.y, Y, fma2(fw, Z, e)));
+  if (COMP)
+    e = fma2(pack2(rf.x, rf.x), lx, fma2(pack2(rf.y, rf.y), ly, fma2(pack2(rf.z, rf.z), lz, e)));
+  const f32x2 f = pack2(__uint_as_float((q[0] >> 9) | 0x3f800000u), __uint_as_float((q[1] >> 9) | 0x3f800000u));
+  sincos2(fma2(f, pack2(K2PI, K2PI), e), c, fr, fi);
+}
+
+constexpr int RM_NONE = VISS_RECON_MASK_NONE, RM_REF = VISS_RECON_MASK_REF, RM_GEO = VISS_RECON_MASK_GEOMETRIC;
 constexpr int REC_SAT_CACHE = 512;   // satellite directions cached per tile (float4)
 constexpr int REC_CONE_CACHE = 128;  // snapshot cones cached per tile
 
 template <int RM, bool COMP, int Q>
-struct RecSmem {
+struct RecSmem {  // unmasked and REF
+  int4 r0[Q];                    // {U, V, W, bias}
+  ulonglong2 r1[Q];              // {fu, fu, fv, fv}
+  ulonglong2 r2[Q];              // {fw, fw, c, c}
+  float4 rf[COMP ? Q : 1];
+  int4 win[RM == RM_REF ? Q : 1];
+  float4 acc[REC_PIX];           // running totals (re, im) and their Kahan compensation per pixel
+};
+
+template <bool COMP, int Q>
+struct RecSmem<RM_GEO, COMP, Q> {
   int4 r0[Q];
   float4 r1[Q];
   float4 rf[COMP ? Q : 1];
-  int4 win[RM == RM_REF ? Q : 1];
-  uint32_t pm[RM == RM_GEO ? Q : 1];   // the row's two satellites as bits of its snapshot's satellites
-  int snap[RM == RM_GEO ? Q : 1];
-  int runend[RM == RM_GEO ? Q : 1];
-  float4 sat[RM == RM_GEO ? REC_SAT_CACHE : 1];
-  float4 cone[RM == RM_GEO ? 2 * REC_CONE_CACHE : 1];
-  float4 wcap[RM == RM_GEO ? 2 * (REC_THREADS / 32) : 1];  // each warp's patch: {axis, cos r}, {sin r}
+  uint32_t pm[Q];   // the row's two satellites as bits of its snapshot's satellites
+  int snap[Q];
+  int runend[Q];
+  float4 sat[REC_SAT_CACHE];
+  float4 cone[2 * REC_CONE_CACHE];
+  float4 wcap[2 * (REC_THREADS / 32)];  // each warp's patch: {axis, cos r}, {sin r}
   int srange[2];
   int wkeep[(REC_THREADS / 32) * ((Q + REC_THREADS - 1) / REC_THREADS)];
-  float4 acc[REC_PIX];            // running totals (re, im) and their Kahan compensation per pixel
+  float4 acc[REC_PIX];
 };
 
+// F = norm * (-fr - i fi)  (the angle carried an extra half turn)
+__device__ __forceinline__ void recon_store(const ReconParams& p, const float4* acc, int64_t j0, float2* out, float norm,
+                                            bool direct) {
+#pragma unroll
+  for (int i = 0; i < REC_TJ; ++i) {
+    const int64_t pos = j0 + i;
+    const float4 t = acc[threadIdx.x * REC_TJ + i];
+    const float fr = t.x, fi = t.y;
+    if (pos < p.J) {
+      if (direct) {
+        const int64_t j = p.perm ? (int64_t)p.perm[pos] : pos;
+        out[j] = make_float2(-fr * norm, -fi * norm);
+      } else {
+        out[pos] = make_float2(fr, fi);
+      }
+    }
+  }
+}
+
+// Unmasked and REF-mask items.  Every FP32 operation of a term but the SFU's runs packed, two pixels
+// at a time, and of integer uvw every fourth term is a polynomial: the FMA pipe has room
+// beside the SFU there (10 of its 16 cycles a warp-term).  What it measured against single
+// operations is at recon_fast_kernel.
 template <int RM, bool FRAC, bool COMP, int Q>
-__device__ __forceinline__ void recon_body(const ReconParams& p, RecSmem<RM, COMP, Q>& sm, int64_t pb, int64_t kb,
+__device__ __forceinline__ void recon_rows(const ReconParams& p, RecSmem<RM, COMP, Q>& sm, int64_t pb, int64_t kb,
+                                           int64_t ke, float2* out, float norm, bool direct) {
+  const int tid = threadIdx.x;
+  const int64_t j0 = pb * REC_PIX + (int64_t)tid * REC_TJ;
+  int A[REC_TJ], B[REC_TJ], C[REC_TJ];
+  // pixels in packed pairs (pixel 2h in the low half, 2h + 1 in the high one)
+  f32x2 XF[REC_TJ / 2], YF[REC_TJ / 2], ZF[REC_TJ / 2];
+  f32x2 LX[REC_TJ / 2], LY[REC_TJ / 2], LZ[REC_TJ / 2];
+  int TP[REC_TJ], PP[REC_TJ];
+  // running totals live in sm.acc
+#pragma unroll
+  for (int i = 0; i < REC_TJ; ++i) {
+    const int64_t pos = j0 + i;  // pixels padded to a whole block
+    const int4 a = p.pix0[pos];
+    A[i] = a.x; B[i] = a.y; C[i] = a.z;
+    TP[i] = PP[i] = -1;
+    if (RM == RM_REF) { const int2 qr = p.pqr[pos]; PP[i] = qr.x; TP[i] = qr.y; }
+    sm.acc[tid * REC_TJ + i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (int h = 0; h < REC_TJ / 2; ++h) {
+    XF[h] = YF[h] = ZF[h] = LX[h] = LY[h] = LZ[h] = 0ull;
+    if (FRAC) {
+      const float4* px = reinterpret_cast<const float4*>(p.pix1) + j0 + 2 * h;
+      const float4 a = px[0], b = px[1];
+      XF[h] = pack2(a.x, b.x); YF[h] = pack2(a.y, b.y); ZF[h] = pack2(a.z, b.z);
+    }
+    if (COMP) {
+      const float4 a = p.plo[j0 + 2 * h], b = p.plo[j0 + 2 * h + 1];
+      LX[h] = pack2(a.x, b.x); LY[h] = pack2(a.y, b.y); LZ[h] = pack2(a.z, b.z);
+    }
+  }
+  const int64_t jfirst = pb * REC_PIX;
+  int64_t jlast = jfirst + REC_PIX - 1;
+  if (jlast > p.J - 1) jlast = p.J - 1;
+
+  for (int64_t tile = kb; tile < ke; tile += Q) {
+    const int nq = (int)((ke - tile) < Q ? (ke - tile) : Q);
+    __syncthreads();
+    bool hit = false;
+    for (int r = tid; r < nq; r += REC_THREADS) {
+      const int64_t k = tile + r;
+      const float4 r1 = p.rows1[k];
+      sm.r0[r] = p.rows0[k];
+      sm.r1[r] = make_ulonglong2(pack2(r1.x, r1.x), pack2(r1.y, r1.y));
+      sm.r2[r] = make_ulonglong2(pack2(r1.z, r1.z), pack2(r1.w, r1.w));
+      if (COMP) sm.rf[r] = p.rowsf[k];
+      if (RM == RM_REF) {
+        const int4 wv = p.win[k];
+        sm.win[r] = wv;
+        if (wv.x >= 1 && wv.y >= 1) {
+          const int64_t lo_idx = (int64_t)p.res + 1, hi_idx = (int64_t)wv.y * p.res + wv.x;
+          if (lo_idx <= jlast && hi_idx >= jfirst) hit = true;
+        }
+      }
+    }
+    const bool masked_tile = __syncthreads_or(hit) != 0;
+    f32x2 tr[REC_TJ / 2], ti[REC_TJ / 2];  // this tile's sums
+#pragma unroll
+    for (int h = 0; h < REC_TJ / 2; ++h) tr[h] = ti[h] = 0ull;
+    static_assert(REC_TJ == 4, "two pixel pairs");
+    // row r with all of the thread's pixels; poly: the second pair without the SFU
+    auto row_term = [&](int r, auto poly) {
+      const int4 r0 = sm.r0[r];
+      const ulonglong2 fuv = FRAC ? sm.r1[r] : make_ulonglong2(0ull, 0ull), fwc = sm.r2[r];
+      const float4 rf = COMP ? sm.rf[r] : make_float4(0.f, 0.f, 0.f, 0.f);
+      rec_term2<FRAC, COMP, false>(r0, fuv, fwc.x, rf, fwc.y, A, B, C, XF[0], YF[0], ZF[0], LX[0], LY[0], LZ[0], tr[0],
+                                   ti[0]);
+      rec_term2<FRAC, COMP, decltype(poly)::value>(r0, fuv, fwc.x, rf, fwc.y, A + 2, B + 2, C + 2, XF[1], YF[1], ZF[1],
+                                                   LX[1], LY[1], LZ[1], tr[1], ti[1]);
+    };
+    if (RM == RM_REF && masked_tile) {
+      for (int r = 0; r < nq; ++r) {
+        const int4 r0 = sm.r0[r], wv = sm.win[r];
+        const ulonglong2 fuv = FRAC ? sm.r1[r] : make_ulonglong2(0ull, 0ull), fwc = sm.r2[r];
+        const float4 rf = COMP ? sm.rf[r] : make_float4(0.f, 0.f, 0.f, 0.f);
+        float c, c_;
+        unpack2(fwc.y, c, c_);
+#pragma unroll
+        for (int h = 0; h < REC_TJ / 2; ++h) {
+          float cm[2];
+#pragma unroll
+          for (int o = 0; o < 2; ++o) {
+            const int i = 2 * h + o;
+            cm[o] = TP[i] >= 1 && TP[i] <= wv.x && PP[i] >= 1 && PP[i] <= wv.y ? 0.f : c;
+          }
+          rec_term2<FRAC, COMP, false>(r0, fuv, fwc.x, rf, pack2(cm[0], cm[1]), A + 2 * h, B + 2 * h, C + 2 * h, XF[h],
+                                       YF[h], ZF[h], LX[h], LY[h], LZ[h], tr[h], ti[h]);
+        }
+      }
+    } else {
+      int r = 0;
+      if (!FRAC && !COMP) {
+        for (; r + 4 <= nq; r += 4) {
+          row_term(r, std::false_type{});
+          row_term(r + 1, std::true_type{});
+          row_term(r + 2, std::false_type{});
+          row_term(r + 3, std::true_type{});
+        }
+      }
+#pragma unroll 2
+      for (; r < nq; ++r) row_term(r, std::false_type{});
+    }
+#pragma unroll
+    for (int h = 0; h < REC_TJ / 2; ++h) {
+      float r[2], im[2];
+      unpack2(tr[h], r[0], r[1]);
+      unpack2(ti[h], im[0], im[1]);
+#pragma unroll
+      for (int o = 0; o < 2; ++o) {
+        float4 t = sm.acc[tid * REC_TJ + 2 * h + o];  // owned by this thread alone
+        kahan_add(t.x, t.z, r[o]);
+        kahan_add(t.y, t.w, im[o]);
+        sm.acc[tid * REC_TJ + 2 * h + o] = t;
+      }
+    }
+  }
+  recon_store(p, sm.acc, j0, out, norm, direct);
+}
+
+// Geometric items.
+template <bool FRAC, bool COMP, int Q>
+__device__ __forceinline__ void recon_geo(const ReconParams& p, RecSmem<RM_GEO, COMP, Q>& sm, int64_t pb, int64_t kb,
                                            int64_t ke, float2* out, float norm, bool direct) {
   constexpr int REC_LOAD = (Q + REC_THREADS - 1) / REC_THREADS;  // tile rows per thread in the load
   const int tid = threadIdx.x;
@@ -83,7 +331,6 @@ __device__ __forceinline__ void recon_body(const ReconParams& p, RecSmem<RM, COM
   int A[REC_TJ], B[REC_TJ], C[REC_TJ];
   float XF[REC_TJ], YF[REC_TJ], ZF[REC_TJ];
   float LX[REC_TJ], LY[REC_TJ], LZ[REC_TJ];
-  int TP[REC_TJ], PP[REC_TJ];
   // running totals live in sm.acc; pixel directions (geometric) are re-read per snapshot run
 #pragma unroll
   for (int i = 0; i < REC_TJ; ++i) {
@@ -97,35 +344,28 @@ __device__ __forceinline__ void recon_body(const ReconParams& p, RecSmem<RM, COM
     }
     LX[i] = LY[i] = LZ[i] = 0.f;
     if (COMP) { const float4 lo = p.plo[pos]; LX[i] = lo.x; LY[i] = lo.y; LZ[i] = lo.z; }
-    TP[i] = PP[i] = -1;
-    if (RM == RM_REF) { const int2 qr = p.pqr[pos]; PP[i] = qr.x; TP[i] = qr.y; }
     sm.acc[tid * REC_TJ + i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   unsigned valid = 0;  // bit i: pixel i of this thread is a real pixel
 #pragma unroll
   for (int i = 0; i < REC_TJ; ++i) valid |= (j0 + i < p.J ? 1u : 0u) << i;
-  const int64_t jfirst = pb * REC_PIX;
-  int64_t jlast = jfirst + REC_PIX - 1;
-  if (jlast > p.J - 1) jlast = p.J - 1;
 
   // geometric: the block's bounding cone {axis, cos r, sin r}; a row whose snapshot
   // hides every pixel of the block is dropped from the tile, for all warps at once
   float4 bc0 = make_float4(0.f, 0.f, 0.f, -2.f);
   float bsin = 1.f;
-  if (RM == RM_GEO) {
-    bc0 = __ldg(p.bcones + 2 * pb);
-    bsin = __ldg(p.bcones + 2 * pb + 1).x;
-    // this warp's patch cap (read and written by this warp only)
-    if ((tid & 31) < 2)
-      sm.wcap[2 * (tid >> 5) + (tid & 31)] = __ldg(p.wcones + 2 * (pb * (REC_THREADS / 32) + (tid >> 5)) + (tid & 31));
-    __syncwarp();
-  }
+  bc0 = __ldg(p.bcones + 2 * pb);
+  bsin = __ldg(p.bcones + 2 * pb + 1).x;
+  // this warp's patch cap (read and written by this warp only)
+  if ((tid & 31) < 2)
+    sm.wcap[2 * (tid >> 5) + (tid & 31)] = __ldg(p.wcones + 2 * (pb * (REC_THREADS / 32) + (tid >> 5)) + (tid & 31));
+  __syncwarp();
 
   for (int64_t tile = kb; tile < ke; tile += Q) {
     int nq = (int)((ke - tile) < Q ? (ke - tile) : Q);
     __syncthreads();
-    if (RM == RM_GEO && tid == 0) { sm.srange[0] = 0x7fffffff; sm.srange[1] = -1; }
-    if (RM == RM_GEO) {
+    if (tid == 0) { sm.srange[0] = 0x7fffffff; sm.srange[1] = -1; }
+    {
       // keep row tid unless its snapshot's all-occluded cone {a, cos ao} holds the whole
       // block: angle(axis, a) + r < ao, i.e. axis.a > cos(ao - r) = cos ao cos r + sin ao sin r
       // (REC_LOAD rows per thread, kept rows compacted in order)
@@ -181,26 +421,10 @@ __device__ __forceinline__ void recon_body(const ReconParams& p, RecSmem<RM, COM
       __syncthreads();
       if (nq == 0) continue;  // the block is hidden from every row of this tile
     }
-    bool hit = false;
-    for (int r = tid; r < (RM == RM_GEO ? 0 : nq); r += REC_THREADS) {
-      const int64_t k = tile + r;
-      sm.r0[r] = p.rows0[k];
-      sm.r1[r] = p.rows1[k];
-      if (COMP) sm.rf[r] = p.rowsf[k];
-      if (RM == RM_REF) {
-        const int4 wv = p.win[k];
-        sm.win[r] = wv;
-        if (wv.x >= 1 && wv.y >= 1) {
-          const int64_t lo_idx = (int64_t)p.res + 1, hi_idx = (int64_t)wv.y * p.res + wv.x;
-          if (lo_idx <= jlast && hi_idx >= jfirst) hit = true;
-        }
-      }
-    }
-    const bool masked_tile = __syncthreads_or(hit) != 0;
     float tr[REC_TJ], ti[REC_TJ];  // this tile's sums
 #pragma unroll
     for (int i = 0; i < REC_TJ; ++i) tr[i] = ti[i] = 0.f;
-    if (RM == RM_GEO) {
+    {
       const int s_lo = sm.srange[0], s_hi = sm.srange[1];
       const int nsn = s_hi - s_lo + 1;
       const bool cached = nsn <= REC_CONE_CACHE && nsn * p.nsat <= REC_SAT_CACHE;
@@ -295,33 +519,6 @@ __device__ __forceinline__ void recon_body(const ReconParams& p, RecSmem<RM, COM
         }
         r = re;
       }
-    } else if (RM == RM_REF && masked_tile) {
-      for (int rr = 0; rr < nq; ++rr) {
-        const int4 r0 = sm.r0[rr];
-        const float4 r1 = sm.r1[rr];
-        float4 rf = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (COMP) rf = sm.rf[rr];
-        const int4 wv = sm.win[rr];
-#pragma unroll
-        for (int i = 0; i < REC_TJ; ++i) {
-          const bool skip = TP[i] >= 1 && TP[i] <= wv.x && PP[i] >= 1 && PP[i] <= wv.y;
-          const float c = skip ? 0.f : r1.w;
-          rec_term<FRAC, COMP>(r0, r1, rf, c, A[i], B[i], C[i], XF[i], YF[i], ZF[i], LX[i], LY[i], LZ[i], tr[i],
-                               ti[i]);
-        }
-      }
-    } else {
-#pragma unroll 2
-      for (int rr = 0; rr < nq; ++rr) {
-        const int4 r0 = sm.r0[rr];
-        const float4 r1 = sm.r1[rr];
-        float4 rf = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (COMP) rf = sm.rf[rr];
-#pragma unroll
-        for (int i = 0; i < REC_TJ; ++i)
-          rec_term<FRAC, COMP>(r0, r1, rf, r1.w, A[i], B[i], C[i], XF[i], YF[i], ZF[i], LX[i], LY[i], LZ[i], tr[i],
-                               ti[i]);
-      }
     }
 #pragma unroll
     for (int i = 0; i < REC_TJ; ++i) {
@@ -331,35 +528,22 @@ __device__ __forceinline__ void recon_body(const ReconParams& p, RecSmem<RM, COM
       sm.acc[tid * REC_TJ + i] = t;
     }
   }
-  // F = norm * (-fr - i fi)  (the angle carried an extra half turn)
-#pragma unroll
-  for (int i = 0; i < REC_TJ; ++i) {
-    const int64_t pos = j0 + i;
-    const float4 t = sm.acc[tid * REC_TJ + i];
-    const float fr = t.x, fi = t.y;
-    if (pos < p.J) {
-      if (direct) {
-        const int64_t j = p.perm ? (int64_t)p.perm[pos] : pos;
-        out[j] = make_float2(-fr * norm, -fi * norm);
-      } else {
-        out[pos] = make_float2(fr, fi);
-      }
-    }
-  }
+  recon_store(p, sm.acc, j0, out, norm, direct);
 }
 
 // Persistent: grid = resident CTAs; each CTA takes the next work item (segment,
 // pixel block) from an atomic counter until none are left.  The counter is
 // reset by the host before the launch; no CTA waits on another.
-// Resident CTAs per SM the instances are compiled for.  The unmasked and REF-mask ones
-// fit in 64 registers (a few spills in the REF one), and a fourth CTA hides their tile
-// barriers better (10 MHz recon: unmasked 168.0 -> 162.4 ms, REF windows 168.3 -> 161.2);
-// the geometric one needs 80 (at 64 it spills in its term loops: 163 -> 177 ms).
-template <int RM>
-constexpr int rec_min_blocks() { return RM != RM_GEO ? VISS_REC_MINB + 1 : VISS_REC_MINB; }
-
+// Resident CTAs per SM the instances are compiled for (rec_ctas).  The unmasked FAST one fits in
+// 64 registers, and a fourth CTA hides its tile barriers better; the others need 80 (at 64 the
+// geometric one spills in its term loops, 10 MHz 163 -> 177 ms, the compensated one 8.44
+// against 7.56 ms on 200,003 x 65,537).  Packed against single operations (262,144 x 196,249,
+// the instances at their best CTAs): unmasked fractional 23.4 -> 22.3 ms, compensated 29.2 -> 27.3
+// (32.6 at four CTAs), integer with every fourth term a polynomial 21.5 -> 21.1, REF windows
+// 21.45 -> 21.26.  The geometric instance gained nothing from them (11.31 -> 11.51 ms on
+// 458,752 x 49,152) and keeps single operations.
 template <int RM, bool COMP, int Q>
-__global__ void __launch_bounds__(REC_THREADS, rec_min_blocks<RM>()) recon_fast_kernel(const ReconParams p) {
+__global__ void __launch_bounds__(REC_THREADS, rec_ctas(RM, COMP)) recon_fast_kernel(const ReconParams p) {
   __shared__ RecSmem<RM, COMP, Q> sm;
   __shared__ int s_item;
   const bool frac = __ldg(p.flags + FLAG_FRAC) != 0;
@@ -374,8 +558,13 @@ __global__ void __launch_bounds__(REC_THREADS, rec_min_blocks<RM>()) recon_fast_
     const int ch = p.seg_ch[seg], slot = p.seg_slot[seg];
     const bool direct = slot < 0;
     float2* out = direct ? p.out + (int64_t)ch * p.J : p.partial + (int64_t)slot * p.J;
-    if (frac) recon_body<RM, true, COMP, Q>(p, sm, pb, p.seg_lo[seg], p.seg_hi[seg], out, p.ch_norm[ch], direct);
-    else recon_body<RM, false, COMP, Q>(p, sm, pb, p.seg_lo[seg], p.seg_hi[seg], out, p.ch_norm[ch], direct);
+    if constexpr (RM == RM_GEO) {
+      if (frac) recon_geo<true, COMP, Q>(p, sm, pb, p.seg_lo[seg], p.seg_hi[seg], out, p.ch_norm[ch], direct);
+      else recon_geo<false, COMP, Q>(p, sm, pb, p.seg_lo[seg], p.seg_hi[seg], out, p.ch_norm[ch], direct);
+    } else {
+      if (frac) recon_rows<RM, true, COMP, Q>(p, sm, pb, p.seg_lo[seg], p.seg_hi[seg], out, p.ch_norm[ch], direct);
+      else recon_rows<RM, false, COMP, Q>(p, sm, pb, p.seg_lo[seg], p.seg_hi[seg], out, p.ch_norm[ch], direct);
+    }
   }
 }
 

@@ -86,6 +86,11 @@ constexpr int RED_GROUPS = 8;
 #define VISS_REC_MINB 3
 #endif
 
+// Resident CTAs per SM of the reconstruction instances (recon.cu).
+constexpr int rec_ctas(int recon_mask, bool comp) {
+  return recon_mask == VISS_RECON_MASK_NONE && !comp ? VISS_REC_MINB + 1 : VISS_REC_MINB;
+}
+
 // Channels of one batched pass, and visibility segments of its reconstruction
 // (their tables travel in the kernel parameters).
 constexpr int VISS_MAX_CH = VISS_MAX_CHANNELS;
