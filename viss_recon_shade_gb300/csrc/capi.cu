@@ -192,8 +192,8 @@ struct RecPlan {
   bool geo = false, ref = false, comp = false, plain = false;
   int4 *pix0 = nullptr, *pix1 = nullptr, *rows0 = nullptr, *win = nullptr;
   float4 *rows1 = nullptr, *plo = nullptr, *pgeo = nullptr, *rowsf = nullptr, *satdir = nullptr, *scones = nullptr;
-  float4 *bcones = nullptr, *wcones = nullptr;
-  int* rowsat = nullptr;
+  float4* wcones = nullptr;
+  int2* rowpm = nullptr;
   int2* pqr = nullptr;
   float2* partial = nullptr;
   float* ratios = nullptr;
@@ -222,13 +222,12 @@ struct RecPlan {
       if (ref) pqr = c.take<int2>(Jpad);
       rows0 = c.take<int4>(Kpad);
       rows1 = c.take<float4>(Kpad);
-      if (geo) rowsat = c.take<int>(Kpad);
+      if (geo) rowpm = c.take<int2>(Kpad);
       if (comp) rowsf = c.take<float4>(Kpad);
       if (ref) win = c.take<int4>(Kpad);
       if (geo) {
         satdir = c.take<float4>(nsd);
         scones = c.take<float4>(2 * S);
-        bcones = c.take<float4>(2 * npb);
         wcones = c.take<float4>(2 * npb * (REC_THREADS / 32));
       }
       if (nslot > 0) partial = c.take<float2>((size_t)nslot * J);
@@ -527,7 +526,7 @@ int recon_impl(const viss_dft_cfg& cfg, const double scale[3], const float dlmn[
   set_scales(pa, scale, cfg.n_offset);
   pa.res = cfg.res; pa.trunc = 0;
   pa.rec0 = p.pix0; pa.rec1 = p.pix1; pa.lo = p.plo; pa.geo = p.pgeo; pa.qr = p.pqr;
-  pa.bcaps = p.bcones; pa.wcaps = p.wcones;
+  pa.wcaps = p.wcones;
   RowPrepArgs ra{};
   ra.u = vis.u; ra.v = vis.v; ra.w = vis.w; ra.wgt = vis.wgt; ra.V = V;
   ra.shade = ratio_arrays ? nullptr : vis.shade;
@@ -536,15 +535,15 @@ int recon_impl(const viss_dft_cfg& cfg, const double scale[3], const float dlmn[
   ra.sn = scale[2]; ra.n_offset = cfg.n_offset;
   ra.ch = bt.ch; ra.padded = false;
   ra.K = vis.K; ra.Kpad = p.Kpad; ra.mask_mode = VISS_MASK_NONE; ra.recon_mask = cfg.recon_mask;
-  ra.rows0 = p.rows0; ra.rows1 = p.rows1; ra.rowsat = p.rowsat; ra.uf = p.rowsf; ra.win = p.win;
+  ra.rows0 = p.rows0; ra.rows1 = p.rows1; ra.rowpm = p.rowpm; ra.uf = p.rowsf; ra.win = p.win;
   ra.flags = p.flags;
   if (p.ref && ratio_arrays)
     for (int i = 0; i < 4; ++i) ra.ratios[i] = ratio_arrays[i];
   if ((rc = launch_prep(pa, ra, p.geo ? sat_args(geo, cfg, p.satdir, p.scones) : SatPrepArgs{}, true, st))) return rc;
   ReconParams rp{};
   rp.pix0 = p.pix0; rp.pix1 = p.pix1; rp.plo = p.plo; rp.pgeo = p.pgeo; rp.pqr = p.pqr;
-  rp.rows0 = p.rows0; rp.rows1 = p.rows1; rp.rowsat = p.rowsat; rp.rowsf = p.rowsf; rp.win = p.win;
-  rp.satdir = p.satdir; rp.scones = p.scones; rp.bcones = p.bcones; rp.wcones = p.wcones;
+  rp.rows0 = p.rows0; rp.rows1 = p.rows1; rp.rowpm = p.rowpm; rp.rowsf = p.rowsf; rp.win = p.win;
+  rp.satdir = p.satdir; rp.scones = p.scones; rp.wcones = p.wcones;
   rp.l = sky.l; rp.m = sky.m; rp.n = sky.n; rp.sat_pos = geo ? geo->sat_pos : nullptr;
   rp.flags = p.flags;
   rp.perm = p.perm;

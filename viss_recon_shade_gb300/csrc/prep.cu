@@ -120,12 +120,10 @@ __device__ __forceinline__ void cap_write(const float4& axis, float c2, float4* 
   out[1] = make_float4(sr, 0.f, 0.f, 0.f);
 }
 
-// The records and, on the way, the caps of each warp's patch of 32 * REC_TJ positions and of each
-// block of REC_PIX: one launch and no second read of the directions (two cap kernels with
-// FP64 cosines and arc cosines took 22 us beside 5 us of records on 2,048-12,288 pixels).
-__device__ void prep_pixels_caps(const PixPrepArgs& a, int block, float4* bcaps, float4* wcaps) {
-  __shared__ float4 s_sum[REC_THREADS / 32];
-  __shared__ float s_c2[REC_THREADS / 32];
+// The records and, on the way, the cap of each warp's patch of 32 * REC_TJ positions: one launch and
+// no second read of the directions (cap kernels with FP64 cosines and arc cosines took 22 us
+// beside 5 us of records on 2,048-12,288 pixels).
+__device__ void prep_pixels_caps(const PixPrepArgs& a, int block, float4* wcaps) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t p0 = (int64_t)block * REC_PIX + warp * 32 * REC_TJ + lane;
   float4 g[REC_TJ];
@@ -142,27 +140,7 @@ __device__ void prep_pixels_caps(const PixPrepArgs& a, int block, float4* bcaps,
   for (int i = 0; i < REC_TJ; ++i)
     if (p0 + 32 * i < a.J) c2 = fmaxf(c2, chord2(wa, g[i]));
   c2 = warp_max(c2);
-  if (lane == 0) {
-    cap_write(wa, c2, wcaps + 2 * ((int64_t)block * (REC_THREADS / 32) + warp));
-    s_sum[warp] = make_float4(sx, sy, sz, 0.f);
-  }
-  __syncthreads();
-  sx = sy = sz = 0.f;
-#pragma unroll
-  for (int w = 0; w < REC_THREADS / 32; ++w) { sx += s_sum[w].x; sy += s_sum[w].y; sz += s_sum[w].z; }
-  const float4 ba = cap_axis(sx, sy, sz);
-  c2 = 0.f;
-#pragma unroll
-  for (int i = 0; i < REC_TJ; ++i)
-    if (p0 + 32 * i < a.J) c2 = fmaxf(c2, chord2(ba, g[i]));
-  c2 = warp_max(c2);
-  if (lane == 0) s_c2[warp] = c2;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int w = 1; w < REC_THREADS / 32; ++w) c2 = fmaxf(c2, s_c2[w]);
-    cap_write(ba, c2, bcaps + 2 * (int64_t)block);
-  }
+  if (lane == 0) cap_write(wa, c2, wcaps + 2 * ((int64_t)block * (REC_THREADS / 32) + warp));
 }
 
 // {min, max} of widx over each run of VIS_P positions (the fine indices a vis
@@ -222,6 +200,7 @@ __device__ __forceinline__ void prep_row(const RowPrepArgs& a, bool recon, int64
     a.rows0[pr] = make_int4(0, 0, 0, PHASE_BIAS);
     a.rows1[pr] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (a.rowsat) a.rowsat[pr] = PAD_PACKED;
+    if (a.rowpm) a.rowpm[pr] = make_int2(0, 1);
     if (a.uf) a.uf[pr] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (a.win) a.win[pr] = recon ? make_int4(0, 0, 0, 0) : make_int4(1, 0, 0, 0);
     return;
@@ -239,14 +218,19 @@ __device__ __forceinline__ void prep_row(const RowPrepArgs& a, bool recon, int64
   }
   if (!ok) atomicOr(a.flags + FLAG_ERR, 1);
   if (frac) atomicOr(a.flags + FLAG_FRAC, 1);
-  if (a.rowsat) {
+  if (a.snap) {
     int packed = PAD_PACKED;
+    int2 sp = make_int2(0, 1);
     const int s = a.snap[k];
     const int pr2 = a.pair[k];
     const int pm = pr2 & 0xffff, pn = (pr2 >> 16) & 0xffff;
     if (s < 0 || s >= a.S || pm >= a.nsat || pn >= a.nsat) atomicOr(a.flags + FLAG_ERR, 2);
-    else packed = (s * a.nsat + pm) | ((pn - pm + 32) << 26);
-    a.rowsat[pr] = packed;
+    else {
+      packed = (s * a.nsat + pm) | ((pn - pm + 32) << 26);
+      sp = make_int2(s, (1 << pm) | (1 << pn));
+    }
+    if (a.rowsat) a.rowsat[pr] = packed;
+    if (a.rowpm) a.rowpm[pr] = sp;
   }
   // PHASE_BIAS plus the per-row part of f_w * z: f_w * sn * n_offset; the
   // reconstruction folds the visibility's phase in too: y e^{ix} = |y| e^{i(x + arg y)}
@@ -391,7 +375,7 @@ __global__ void __launch_bounds__(PREP_THREADS) prep_kernel(const PixPrepArgs pi
                                                             int pix_blocks, int row_blocks, bool recon) {
   int b = (int)blockIdx.x;
   if (b < pix_blocks) {
-    if (CAPS) prep_pixels_caps(pix, b, pix.bcaps, pix.wcaps);
+    if (CAPS) prep_pixels_caps(pix, b, pix.wcaps);
     else {
       const int64_t pos = (int64_t)b * PREP_THREADS + threadIdx.x;
       if (pos < pix.Jpad) prep_pixel(pix, pos);
@@ -410,7 +394,7 @@ __global__ void __launch_bounds__(PREP_THREADS) prep_kernel(const PixPrepArgs pi
 static int64_t prep_blocks(int64_t n) { return (n + PREP_THREADS - 1) / PREP_THREADS; }
 
 int launch_prep(const PixPrepArgs& pix, const RowPrepArgs& row, SatPrepArgs sat, bool recon, cudaStream_t st) {
-  const bool caps = pix.bcaps != nullptr;
+  const bool caps = pix.wcaps != nullptr;
   const int64_t np = caps ? pix.Jpad / REC_PIX : prep_blocks(pix.Jpad), nr = prep_blocks(row.Kpad);
   int64_t ns = 0;
   if (sat.S > 0 && sat.nsat > 0) {

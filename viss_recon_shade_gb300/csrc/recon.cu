@@ -3,26 +3,24 @@
 //
 // F_j = norm * sum_k [not masked] y_k exp(+2 pi i t_kj),  y_k = wgt_k V_k
 //
-// A work item is REC_PIX = 1024 pixels (4 per thread, fixed-point coordinates
-// in registers) against one segment of visibility rows of one channel, streamed
-// through shared memory in tiles of 2 REC_Q rows, 4 REC_Q with the geometric mask and
-// no compensation (REC_Q or REC_Q / 2 on request).
+// A work item of the unmasked and REF kernels is REC_PIX = 1024 pixels (4 per thread,
+// fixed-point coordinates in registers) against one segment of visibility rows of one
+// channel, streamed through shared memory in tiles of 2 REC_Q rows (REC_Q or REC_Q / 2 on
+// request); one of the geometric kernel is a warp's 128 pixels against such a segment.
 // The phase of y_k is folded into the
 // row's fixed-point bias (y e^{ix} = |y| e^{i(x + arg y)}), so a term is the
 // same as in the vis kernel: 3 IMAD [+3 FFMA fractional uvw] [+3 FFMA
 // compensated], turns -> angle, __sincosf, 2 FFMA with |y_k|.
 // Masks:
-//   GEOMETRIC: rows hidden from the whole pixel block are dropped when a tile is
-//     loaded; the rest come in snapshot runs.  Per run the warp tests the cap
-//     bounding its 128 pixels against the snapshot's cones (warp-uniform); where
-//     that leaves the run open, every thread tests its pixels against the
-//     snapshot's bounding cone and the warp votes: all occluded -> the run is
-//     skipped, all visible -> unmasked loop, else the thread builds a per-pixel
-//     satellite occlusion bitmask and tests each row's pair.
+//   GEOMETRIC: a lane tests its row's snapshot cones against the cap bounding the warp's
+//     128 pixels: rows hidden from all of them are dropped, rows that all of them see run
+//     unmasked.  For a snapshot that this leaves open, every thread tests its pixels
+//     against the cones and the warp votes; if that leaves it open too, the thread builds a
+//     per-pixel satellite occlusion bitmask and tests each row's pair.
 //   REF: the reference ratio mask can only fire on pixels (thetaP, phiP) with
 //     1 <= thetaP <= tmax_k, 1 <= phiP <= pmax_k; tiles whose rows cannot touch
 //     the item's pixels run unmasked.
-// Persistent CTAs take items from an atomic counter, longest segments first.
+// Persistent CTAs (geometric: warps) take items from an atomic counter, longest segments first.
 // A channel split into several segments leaves partial sums per segment,
 // reduced in a fixed order.
 #include <type_traits>
@@ -145,9 +143,7 @@ __device__ __forceinline__ void rec_term2(const int4& r0, const ulonglong2& fuv,
   sincos2(fma2(f, pack2(K2PI, K2PI), e), c, fr, fi);
 }
 
-constexpr int RM_NONE = VISS_RECON_MASK_NONE, RM_REF = VISS_RECON_MASK_REF, RM_GEO = VISS_RECON_MASK_GEOMETRIC;
-constexpr int REC_SAT_CACHE = 512;   // satellite directions cached per tile (float4)
-constexpr int REC_CONE_CACHE = 128;  // snapshot cones cached per tile
+constexpr int RM_NONE = VISS_RECON_MASK_NONE, RM_REF = VISS_RECON_MASK_REF;
 
 template <int RM, bool COMP, int Q>
 struct RecSmem {  // unmasked and REF
@@ -157,22 +153,6 @@ struct RecSmem {  // unmasked and REF
   float4 rf[COMP ? Q : 1];
   int4 win[RM == RM_REF ? Q : 1];
   float4 acc[REC_PIX];           // running totals (re, im) and their Kahan compensation per pixel
-};
-
-template <bool COMP, int Q>
-struct RecSmem<RM_GEO, COMP, Q> {
-  int4 r0[Q];
-  float4 r1[Q];
-  float4 rf[COMP ? Q : 1];
-  uint32_t pm[Q];   // the row's two satellites as bits of its snapshot's satellites
-  int snap[Q];
-  int runend[Q];
-  float4 sat[REC_SAT_CACHE];
-  float4 cone[2 * REC_CONE_CACHE];
-  float4 wcap[2 * (REC_THREADS / 32)];  // each warp's patch: {axis, cos r}, {sin r}
-  int srange[2];
-  int wkeep[(REC_THREADS / 32) * ((Q + REC_THREADS - 1) / REC_THREADS)];
-  float4 acc[REC_PIX];
 };
 
 // F = norm * (-fr - i fi)  (the angle carried an extra half turn)
@@ -319,22 +299,45 @@ __device__ __forceinline__ void recon_rows(const ReconParams& p, RecSmem<RM, COM
   recon_store(p, sm.acc, j0, out, norm, direct);
 }
 
-// Geometric items.
-template <bool FRAC, bool COMP, int Q>
-__device__ __forceinline__ void recon_geo(const ReconParams& p, RecSmem<RM_GEO, COMP, Q>& sm, int64_t pb, int64_t kb,
-                                           int64_t ke, float2* out, float norm, bool direct) {
-  constexpr int REC_LOAD = (Q + REC_THREADS - 1) / REC_THREADS;  // tile rows per thread in the load
-  const int tid = threadIdx.x;
-  // a warp owns 32 * REC_TJ consecutive positions: with the spatial order of
-  // the geometric passes that is one compact patch of sky
-  const int64_t j0 = pb * REC_PIX + (int64_t)tid * REC_TJ;
+// Geometric items: a warp's own patch of 32 * REC_TJ positions against one segment.  With the
+// spatial order of the geometric passes a patch is one compact piece of sky, so most snapshots
+// hide or show it as a whole.  Bound by the SFU (16 cycles a warp-term) and register reads
+// (15) as the other kernels are, but what a pass computes differs from warp to warp: a block
+// that shares its row tiles waits at their barriers for the warp that sees the most (a third of
+// the stalls on 28,672 x 12,288).  So nothing is shared: a warp stages 32 rows at a time in its
+// own corner of shared memory (64 or 128 at a time: 1.2 and 1 % slower on 10 MHz), and one
+// snapshot's bits are kept there for as long as it stays open.  Rows of an open snapshot
+// whose satellites hide the whole patch are skipped.  Against blocks with shared row tiles:
+// 3,360 x 2,048 19.8 -> 16.6 us, 28,672 x 12,288 254 -> 210 us, 458,752 x 49,152 11.28 -> 10.47 ms,
+// 1,835,008 x 196,608 157.2 -> 150.1 ms (rows as 64-bit indexes: 152.4, they spill).  Tried: the
+// packed terms of the other kernels (10 MHz +3 %), halves of a patch skipped by themselves
+// (+1 to 4 %).
+struct GeoWarp {
+  int4 r0[32];
+  float4 r1[32];
+  uint32_t pm[32];          // the row's two satellites as bits of its snapshot's satellites
+  float4 sat[32];           // the open snapshot's satellite directions
+  uint32_t bits[REC_TJ][32];  // per pixel: the open snapshot's satellites that it is hidden from
+  float4 acc[32 * REC_TJ];  // running totals (re, im) and their Kahan compensation per pixel
+};
+template <bool COMP>
+struct GeoSmem {
+  GeoWarp w[REC_THREADS / 32];
+  float4 rf[COMP ? REC_THREADS : 1];
+};
+
+template <bool FRAC, bool COMP>
+__device__ __forceinline__ void recon_geo(const ReconParams& p, GeoWarp& sm, float4* rfs, unsigned patch, unsigned kb,
+                                          unsigned ke, float2* out, float norm, bool direct) {
+  const int lane = threadIdx.x & 31;
+  // J <= 2^30 and K <= 2^31: 32-bit positions and rows; pixel i stands at j0 + 32 i
+  const unsigned j0 = patch * (32 * REC_TJ) + lane, nj = (unsigned)p.J;
   int A[REC_TJ], B[REC_TJ], C[REC_TJ];
   float XF[REC_TJ], YF[REC_TJ], ZF[REC_TJ];
   float LX[REC_TJ], LY[REC_TJ], LZ[REC_TJ];
-  // running totals live in sm.acc; pixel directions (geometric) are re-read per snapshot run
 #pragma unroll
   for (int i = 0; i < REC_TJ; ++i) {
-    const int64_t pos = j0 + i;  // pixels padded to a whole block
+    const unsigned pos = j0 + 32 * i;  // pixels padded to a whole block
     const int4 a = p.pix0[pos];
     A[i] = a.x; B[i] = a.y; C[i] = a.z;
     XF[i] = YF[i] = ZF[i] = 0.f;
@@ -344,191 +347,172 @@ __device__ __forceinline__ void recon_geo(const ReconParams& p, RecSmem<RM_GEO, 
     }
     LX[i] = LY[i] = LZ[i] = 0.f;
     if (COMP) { const float4 lo = p.plo[pos]; LX[i] = lo.x; LY[i] = lo.y; LZ[i] = lo.z; }
-    sm.acc[tid * REC_TJ + i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    sm.acc[32 * i + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  unsigned valid = 0;  // bit i: pixel i of this thread is a real pixel
-#pragma unroll
-  for (int i = 0; i < REC_TJ; ++i) valid |= (j0 + i < p.J ? 1u : 0u) << i;
-
-  // geometric: the block's bounding cone {axis, cos r, sin r}; a row whose snapshot
-  // hides every pixel of the block is dropped from the tile, for all warps at once
-  float4 bc0 = make_float4(0.f, 0.f, 0.f, -2.f);
-  float bsin = 1.f;
-  bc0 = __ldg(p.bcones + 2 * pb);
-  bsin = __ldg(p.bcones + 2 * pb + 1).x;
-  // this warp's patch cap (read and written by this warp only)
-  if ((tid & 31) < 2)
-    sm.wcap[2 * (tid >> 5) + (tid & 31)] = __ldg(p.wcones + 2 * (pb * (REC_THREADS / 32) + (tid >> 5)) + (tid & 31));
-  __syncwarp();
-
-  for (int64_t tile = kb; tile < ke; tile += Q) {
-    int nq = (int)((ke - tile) < Q ? (ke - tile) : Q);
-    __syncthreads();
-    if (tid == 0) { sm.srange[0] = 0x7fffffff; sm.srange[1] = -1; }
-    {
-      // keep row tid unless its snapshot's all-occluded cone {a, cos ao} holds the whole
-      // block: angle(axis, a) + r < ao, i.e. axis.a > cos(ao - r) = cos ao cos r + sin ao sin r
-      // (REC_LOAD rows per thread, kept rows compacted in order)
-      bool keep[REC_LOAD];
-      int pk[REC_LOAD];
-      unsigned bal[REC_LOAD];
-#pragma unroll
-      for (int h = 0; h < REC_LOAD; ++h) {
-        const int r = h * REC_THREADS + tid;
-        keep[h] = false;
-        pk[h] = 0;
-        if (r < nq) {
-          pk[h] = p.rowsat[tile + r];
-          const int sn = sat_gm(pk[h]) / p.nsat;
-          const float4 sc = __ldg(p.scones + 2 * (int64_t)sn);
-          keep[h] = true;
-          if (sc.w <= 1.f && bc0.w >= -1.f && sc.w < bc0.w) {  // the cone is wider than the block
-            const float cao = sc.w, sao = sqrtf(fmaxf(0.f, 1.f - cao * cao));
-            const float lim = fmaf(cao, bc0.w, sao * bsin) + 1e-5f;
-            const float d = fmaf(bc0.x, sc.x, fmaf(bc0.y, sc.y, bc0.z * sc.z));
-            keep[h] = !(d > lim);
-          }
-        }
-        bal[h] = __ballot_sync(0xffffffffu, keep[h]);
-        if ((tid & 31) == 0) sm.wkeep[h * (REC_THREADS / 32) + (tid >> 5)] = __popc(bal[h]);
-      }
-      __syncthreads();
-      int base = 0;
-#pragma unroll
-      for (int h = 0; h < REC_LOAD; ++h) {
-        int off = base + __popc(bal[h] & ((1u << (tid & 31)) - 1u)), tot = 0;
-#pragma unroll
-        for (int w2 = 0; w2 < REC_THREADS / 32; ++w2) {
-          const int c = sm.wkeep[h * (REC_THREADS / 32) + w2];
-          if (w2 < (tid >> 5)) off += c;
-          tot += c;
-        }
-        if (keep[h]) {
-          const int64_t k = tile + h * REC_THREADS + tid;
-          sm.r0[off] = p.rows0[k];
-          sm.r1[off] = p.rows1[k];
-          if (COMP) sm.rf[off] = p.rowsf[k];
-          const int sn = sat_gm(pk[h]) / p.nsat;
-          const int g0 = sn * p.nsat;
-          sm.pm[off] = (1u << (sat_gm(pk[h]) - g0)) | (1u << (sat_gn(pk[h]) - g0));
-          sm.snap[off] = sn;
-          atomicMin(&sm.srange[0], sn);
-          atomicMax(&sm.srange[1], sn);
-        }
-        base += tot;
-      }
-      nq = base;
-      __syncthreads();
-      if (nq == 0) continue;  // the block is hidden from every row of this tile
-    }
+  int open = -1;         // the snapshot whose bits are in sm.bits
+  uint32_t hides = 0u;   // its satellites that hide the whole patch
+  for (unsigned tile = kb; tile < ke; tile += REC_Q) {
+    const unsigned te = min(tile + REC_Q, ke);
     float tr[REC_TJ], ti[REC_TJ];  // this tile's sums
 #pragma unroll
     for (int i = 0; i < REC_TJ; ++i) tr[i] = ti[i] = 0.f;
-    {
-      const int s_lo = sm.srange[0], s_hi = sm.srange[1];
-      const int nsn = s_hi - s_lo + 1;
-      const bool cached = nsn <= REC_CONE_CACHE && nsn * p.nsat <= REC_SAT_CACHE;
-      if (cached) {
-        for (int t = tid; t < nsn * p.nsat; t += REC_THREADS) sm.sat[t] = p.satdir[(int64_t)s_lo * p.nsat + t];
-        for (int t = tid; t < 2 * nsn; t += REC_THREADS) sm.cone[t] = p.scones[2 * (int64_t)s_lo + t];
-      }
-      for (int r = tid; r < nq; r += REC_THREADS) {
-        const int sn = sm.snap[r];
-        if (r == 0 || sm.snap[r - 1] != sn) {
-          int e = r + 1;
-          while (e < nq && sm.snap[e] == sn) ++e;
-          sm.runend[r] = e;
-        }
-      }
-      __syncthreads();
-      for (int r = 0; r < nq;) {
-        const int re = sm.runend[r];
-        const int sn = sm.snap[r];
-        const float4 c0 = cached ? sm.cone[2 * (sn - s_lo)] : __ldg(p.scones + 2 * (int64_t)sn);
-        const float4 c1 = cached ? sm.cone[2 * (sn - s_lo) + 1] : __ldg(p.scones + 2 * (int64_t)sn + 1);
-        // The warp's patch cap {a, r} against the snapshot's cones (warp-uniform):
-        // all hidden when angle(a, c) + r < alpha_occ, i.e. a.c > cos(alpha_occ - r);
-        // all visible when angle(a, c) - r > alpha_vis, i.e. a.c < cos(alpha_vis + r)
-        // (alpha_vis + r < pi).  Margins of 1e-5 in the cosine; what the cap leaves
-        // open the per-pixel vote decides, so the decisions are the vote's.
-        const float4 wc = sm.wcap[2 * (tid >> 5)];
-        const float ws = sm.wcap[2 * (tid >> 5) + 1].x;
+    for (unsigned b = tile; b < te; b += 32) {
+      // each lane decides its row's snapshot against the patch's cap {a, r}:
+      // all hidden when angle(a, c) + r < alpha_occ, i.e. a.c > cos(alpha_occ - r);
+      // all visible when angle(a, c) - r > alpha_vis, i.e. a.c < cos(alpha_vis + r)
+      // (alpha_vis + r < pi).  Margins of 1e-5 in the cosine.
+      bool hid = true, vis = false;
+      int sn = -1;
+      __syncwarp();  // the last batch's rows are consumed
+      if (b + lane < te) {
+        const int2 sp = p.rowpm[b + lane];
+        sn = sp.x;
+        const float4 wc = __ldg(p.wcones + 2 * patch);
+        const float ws = __ldg(p.wcones + 2 * patch + 1).x;
+        const float4 c0 = __ldg(p.scones + 2 * (unsigned)sn), c1 = __ldg(p.scones + 2 * (unsigned)sn + 1);
         const float dw = fmaf(wc.x, c0.x, fmaf(wc.y, c0.y, wc.z * c0.z));
-        bool wocc = false, wvis = false;
+        hid = false;
         if (wc.w >= -1.f) {
-          wocc = c0.w <= 1.f && c0.w < wc.w && dw > fmaf(c0.w, wc.w, c1.y * ws) + 1e-5f;
-          wvis = c1.x >= -1.f && fmaf(c1.z, wc.w, c1.x * ws) > 0.f && dw < fmaf(c1.x, wc.w, -c1.z * ws) - 1e-5f;
+          hid = c0.w <= 1.f && c0.w < wc.w && dw > fmaf(c0.w, wc.w, c1.y * ws) + 1e-5f;
+          vis = c1.x >= -1.f && fmaf(c1.z, wc.w, c1.x * ws) > 0.f && dw < fmaf(c1.x, wc.w, -c1.z * ws) - 1e-5f;
         }
-        if (!wocc && !wvis) {
-          bool all_vis = true, all_occ = true;
-#pragma unroll
-          for (int i = 0; i < REC_TJ; ++i) {
-            const float4 g = __ldg(p.pgeo + j0 + i);
-            const float d = fmaf(g.x, c0.x, fmaf(g.y, c0.y, g.z * c0.z));
-            const bool v = (valid >> i) & 1u;
-            all_vis &= !v || d < c1.x;
-            all_occ &= !v || d > c0.w;
-          }
-          wocc = __all_sync(0xffffffffu, all_occ);
-          wvis = __all_sync(0xffffffffu, all_vis);
+        if (!hid) {
+          sm.r0[lane] = p.rows0[b + lane];
+          sm.r1[lane] = p.rows1[b + lane];
+          if (COMP) rfs[lane] = p.rowsf[b + lane];
+          sm.pm[lane] = (uint32_t)sp.y;
         }
-        if (wocc) { r = re; continue; }
-        if (wvis) {
+      }
+      unsigned todo = __ballot_sync(0xffffffffu, !hid);
+      unsigned seen = __ballot_sync(0xffffffffu, vis);
+      __syncwarp();
+      while (todo) {
+        const int r = __ffs(todo) - 1;
+        if ((seen >> r) & 1u) {
+          // a run of rows that see the whole patch
+          const unsigned gap = ~((todo & seen) >> r);
+          const int re = gap ? r + __ffs(gap) - 1 : 32;
+          todo &= re < 32 ? 0xffffffffu << re : 0u;
 #pragma unroll 2
           for (int rr = r; rr < re; ++rr) {
             const int4 r0 = sm.r0[rr];
             const float4 r1 = sm.r1[rr];
             float4 rf = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (COMP) rf = sm.rf[rr];
+            if (COMP) rf = rfs[rr];
 #pragma unroll
             for (int i = 0; i < REC_TJ; ++i)
               rec_term<FRAC, COMP>(r0, r1, rf, r1.w, A[i], B[i], C[i], XF[i], YF[i], ZF[i], LX[i], LY[i], LZ[i],
                                    tr[i], ti[i]);
           }
-        } else {
-          // per-pixel satellite occlusion bits for snapshot sn
-          uint32_t bits[REC_TJ];
-          const int g0 = sn * p.nsat;
-#pragma unroll
-          for (int i = 0; i < REC_TJ; ++i) bits[i] = 0u;
+          continue;
+        }
+        // the batch's rows of one snapshot that the cap leaves open: the pixels vote
+        const int s = __shfl_sync(0xffffffffu, sn, r);
+        const unsigned same = __ballot_sync(0xffffffffu, sn == s) & todo;
+        if (s != open) {
+          open = s;
+          const float4 c0 = __ldg(p.scones + 2 * (unsigned)s), c1 = __ldg(p.scones + 2 * (unsigned)s + 1);
+          bool all_vis = true, all_occ = true;
 #pragma unroll
           for (int i = 0; i < REC_TJ; ++i) {
-            const float4 g = __ldg(p.pgeo + j0 + i);
-            for (int sat = 0; sat < p.nsat; ++sat) {
-              const float4 d = cached ? sm.sat[(sn - s_lo) * p.nsat + sat] : __ldg(p.satdir + g0 + sat);
-              const float e = fmaf(g.x, d.x, fmaf(g.y, d.y, fmaf(g.z, d.z, d.w)));
-              bool occ = e < 0.f;
-              if (fabsf(e) < GEO_EPS && ((valid >> i) & 1u)) occ = geo_exact_pix(p, __float_as_int(g.w), g0 + sat);
-              bits[i] |= (occ ? 1u : 0u) << sat;
-            }
+            const float4 g = __ldg(p.pgeo + j0 + 32 * i);
+            const float d = fmaf(g.x, c0.x, fmaf(g.y, c0.y, g.z * c0.z));
+            const bool v = j0 + 32 * i < nj;
+            all_vis &= !v || d < c1.x;
+            all_occ &= !v || d > c0.w;
           }
-#pragma unroll 2
-          for (int rr = r; rr < re; ++rr) {
-            const int4 r0 = sm.r0[rr];
-            const float4 r1 = sm.r1[rr];
-            float4 rf = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (COMP) rf = sm.rf[rr];
-            const uint32_t pm = sm.pm[rr];
+          all_occ = __all_sync(0xffffffffu, all_occ);
+          all_vis = __all_sync(0xffffffffu, all_vis);
+          hides = all_occ ? 0xffffffffu : 0u;
+          if (all_occ || all_vis) {
 #pragma unroll
+            for (int i = 0; i < REC_TJ; ++i) sm.bits[i][lane] = hides;
+          } else {
+            // per-pixel satellite occlusion bits for snapshot s
+            if (lane < p.nsat) sm.sat[lane] = __ldg(p.satdir + s * p.nsat + lane);
+            __syncwarp();
+            hides = 0xffffffffu;
+#pragma unroll 1
             for (int i = 0; i < REC_TJ; ++i) {
-              const float c = (bits[i] & pm) ? 0.f : r1.w;
-              rec_term<FRAC, COMP>(r0, r1, rf, c, A[i], B[i], C[i], XF[i], YF[i], ZF[i], LX[i], LY[i], LZ[i],
-                                   tr[i], ti[i]);
+              const float4 g = __ldg(p.pgeo + j0 + 32 * i);
+              const bool v = j0 + 32 * i < nj;
+              uint32_t bits = 0u;
+#pragma unroll 4
+              for (int sat = 0; sat < p.nsat; ++sat) {
+                const float4 d = sm.sat[sat];
+                const float e = fmaf(g.x, d.x, fmaf(g.y, d.y, fmaf(g.z, d.z, d.w)));
+                bool occ = e < 0.f;
+                if (fabsf(e) < GEO_EPS && v) occ = geo_exact_pix(p, __float_as_int(g.w), s * p.nsat + sat);
+                bits |= (occ ? 1u : 0u) << sat;
+              }
+              sm.bits[i][lane] = bits;
+              if (v) hides &= bits;
             }
+            __syncwarp();
+            hides = __reduce_and_sync(0xffffffffu, hides);
           }
         }
-        r = re;
+        todo &= ~same;
+        uint32_t bits[REC_TJ];
+#pragma unroll
+        for (int i = 0; i < REC_TJ; ++i) bits[i] = sm.bits[i][lane];
+        // a row whose satellites hide the whole patch is skipped
+        for (unsigned m = __ballot_sync(0xffffffffu, !(sm.pm[lane] & hides)) & same; m; m &= m - 1) {
+          const int rr = __ffs(m) - 1;
+          const int4 r0 = sm.r0[rr];
+          const float4 r1 = sm.r1[rr];
+          float4 rf = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (COMP) rf = rfs[rr];
+          const uint32_t pm = sm.pm[rr];
+#pragma unroll
+          for (int i = 0; i < REC_TJ; ++i) {
+            const float c = (bits[i] & pm) ? 0.f : r1.w;
+            rec_term<FRAC, COMP>(r0, r1, rf, c, A[i], B[i], C[i], XF[i], YF[i], ZF[i], LX[i], LY[i], LZ[i],
+                                 tr[i], ti[i]);
+          }
+        }
       }
     }
 #pragma unroll
     for (int i = 0; i < REC_TJ; ++i) {
-      float4 t = sm.acc[tid * REC_TJ + i];  // owned by this thread alone
+      float4 t = sm.acc[32 * i + lane];  // owned by this thread alone
       kahan_add(t.x, t.z, tr[i]);
       kahan_add(t.y, t.w, ti[i]);
-      sm.acc[tid * REC_TJ + i] = t;
+      sm.acc[32 * i + lane] = t;
     }
   }
-  recon_store(p, sm.acc, j0, out, norm, direct);
+  // F = norm * (-fr - i fi)  (the angle carried an extra half turn)
+#pragma unroll
+  for (int i = 0; i < REC_TJ; ++i) {
+    const unsigned pos = j0 + 32 * i;
+    const float4 t = sm.acc[32 * i + lane];
+    if (pos < nj) {
+      if (direct) out[p.perm ? (unsigned)p.perm[pos] : pos] = make_float2(-t.x * norm, -t.y * norm);
+      else out[pos] = make_float2(t.x, t.y);
+    }
+  }
+}
+
+template <bool COMP>
+__global__ void __launch_bounds__(REC_THREADS, rec_ctas(VISS_RECON_MASK_GEOMETRIC, COMP)) recon_geo_kernel(const ReconParams p) {
+  __shared__ GeoSmem<COMP> sm;
+  const bool frac = __ldg(p.flags + FLAG_FRAC) != 0;
+  const int warp = threadIdx.x >> 5;
+  const unsigned npatch = (unsigned)((p.J + 32 * REC_TJ - 1) / (32 * REC_TJ));
+  for (;;) {
+    unsigned item = 0;  // up to VISS_MAX_SEG * 2^23
+    if ((threadIdx.x & 31) == 0) item = (unsigned)atomicAdd(p.flags + FLAG_REC_COUNTER, 1);
+    item = __shfl_sync(0xffffffffu, item, 0);
+    const unsigned seg = item / npatch;
+    if (seg >= (unsigned)p.nseg) break;
+    const unsigned patch = item - seg * npatch;
+    const int ch = p.seg_ch[seg], slot = p.seg_slot[seg];
+    const bool direct = slot < 0;
+    float2* out = direct ? p.out + (int64_t)ch * p.J : p.partial + (int64_t)slot * p.J;
+    float4* rf = sm.rf + (COMP ? 32 * warp : 0);
+    if (frac) recon_geo<true, COMP>(p, sm.w[warp], rf, patch, (unsigned)p.seg_lo[seg], (unsigned)p.seg_hi[seg], out, p.ch_norm[ch], direct);
+    else recon_geo<false, COMP>(p, sm.w[warp], rf, patch, (unsigned)p.seg_lo[seg], (unsigned)p.seg_hi[seg], out, p.ch_norm[ch], direct);
+  }
 }
 
 // Persistent: grid = resident CTAs; each CTA takes the next work item (segment,
@@ -536,12 +520,11 @@ __device__ __forceinline__ void recon_geo(const ReconParams& p, RecSmem<RM_GEO, 
 // reset by the host before the launch; no CTA waits on another.
 // Resident CTAs per SM the instances are compiled for (rec_ctas).  The unmasked FAST one fits in
 // 64 registers, and a fourth CTA hides its tile barriers better; the others need 80 (at 64 the
-// geometric one spills in its term loops, 10 MHz 163 -> 177 ms, the compensated one 8.44
-// against 7.56 ms on 200,003 x 65,537).  Packed against single operations (262,144 x 196,249,
+// geometric one spills, 10 MHz 155 -> 167 ms, the compensated one 8.44 against 7.56 ms on
+// 200,003 x 65,537).  Packed against single operations (262,144 x 196,249,
 // the instances at their best CTAs): unmasked fractional 23.4 -> 22.3 ms, compensated 29.2 -> 27.3
 // (32.6 at four CTAs), integer with every fourth term a polynomial 21.5 -> 21.1, REF windows
-// 21.45 -> 21.26.  The geometric instance gained nothing from them (11.31 -> 11.51 ms on
-// 458,752 x 49,152) and keeps single operations.
+// 21.45 -> 21.26.
 template <int RM, bool COMP, int Q>
 __global__ void __launch_bounds__(REC_THREADS, rec_ctas(RM, COMP)) recon_fast_kernel(const ReconParams p) {
   __shared__ RecSmem<RM, COMP, Q> sm;
@@ -558,13 +541,8 @@ __global__ void __launch_bounds__(REC_THREADS, rec_ctas(RM, COMP)) recon_fast_ke
     const int ch = p.seg_ch[seg], slot = p.seg_slot[seg];
     const bool direct = slot < 0;
     float2* out = direct ? p.out + (int64_t)ch * p.J : p.partial + (int64_t)slot * p.J;
-    if constexpr (RM == RM_GEO) {
-      if (frac) recon_geo<true, COMP, Q>(p, sm, pb, p.seg_lo[seg], p.seg_hi[seg], out, p.ch_norm[ch], direct);
-      else recon_geo<false, COMP, Q>(p, sm, pb, p.seg_lo[seg], p.seg_hi[seg], out, p.ch_norm[ch], direct);
-    } else {
-      if (frac) recon_rows<RM, true, COMP, Q>(p, sm, pb, p.seg_lo[seg], p.seg_hi[seg], out, p.ch_norm[ch], direct);
-      else recon_rows<RM, false, COMP, Q>(p, sm, pb, p.seg_lo[seg], p.seg_hi[seg], out, p.ch_norm[ch], direct);
-    }
+    if (frac) recon_rows<RM, true, COMP, Q>(p, sm, pb, p.seg_lo[seg], p.seg_hi[seg], out, p.ch_norm[ch], direct);
+    else recon_rows<RM, false, COMP, Q>(p, sm, pb, p.seg_lo[seg], p.seg_hi[seg], out, p.ch_norm[ch], direct);
   }
 }
 
@@ -574,25 +552,25 @@ static void launch_tile(const ReconParams& p, int ctas_per_sm, cudaStream_t st) 
   recon_fast_kernel<RM, COMP, Q><<<g, REC_THREADS, 0, st>>>(p);
 }
 
-// Row tiles of 2 REC_Q visibilities (the default; 4 REC_Q for the geometric mask without
-// compensation), REC_Q or REC_Q / 2 (tuning).  Longer geometric tiles meet at the block
-// barrier half as often and drop more hidden rows per load (10 MHz recon 163.0 -> 161.1
-// ms; the satellite cache is halved to keep three CTAs per SM: 37 snapshots of 8
-// satellites fit).  The compensated instance keeps 2 REC_Q: at 4 REC_Q its shared
-// memory would leave two CTAs per SM.
+// Row tiles of 2 REC_Q visibilities (the default), REC_Q or REC_Q / 2 (tuning).
 template <int RM>
 static void launch_rm(const ReconParams& p, int ctas_per_sm, bool comp, cudaStream_t st) {
-  constexpr int QD = RM == RM_GEO ? 4 * REC_Q : 2 * REC_Q;
   if (p.row_tile == 1) {
     if (comp) launch_tile<RM, true, REC_Q / 2>(p, ctas_per_sm, st);
     else launch_tile<RM, false, REC_Q / 2>(p, ctas_per_sm, st);
   } else if (p.row_tile == 2) {
     if (comp) launch_tile<RM, true, 2 * REC_Q>(p, ctas_per_sm, st);
-    else launch_tile<RM, false, QD>(p, ctas_per_sm, st);
+    else launch_tile<RM, false, 2 * REC_Q>(p, ctas_per_sm, st);
   } else {
     if (comp) launch_tile<RM, true, REC_Q>(p, ctas_per_sm, st);
     else launch_tile<RM, false, REC_Q>(p, ctas_per_sm, st);
   }
+}
+
+template <bool COMP>
+static void launch_geo(const ReconParams& p, int ctas_per_sm, cudaStream_t st) {
+  const int g = persistent_grid(recon_geo_kernel<COMP>, REC_THREADS, ctas_per_sm, p.nitems);
+  recon_geo_kernel<COMP><<<g, REC_THREADS, 0, st>>>(p);
 }
 
 int launch_recon_fast(const ReconParams& p, int ctas_per_sm, bool comp, cudaStream_t st) {
@@ -600,7 +578,10 @@ int launch_recon_fast(const ReconParams& p, int ctas_per_sm, bool comp, cudaStre
   switch (p.recon_mask) {
     case VISS_RECON_MASK_NONE: launch_rm<RM_NONE>(p, ctas_per_sm, comp, st); break;
     case VISS_RECON_MASK_REF: launch_rm<RM_REF>(p, ctas_per_sm, comp, st); break;
-    case VISS_RECON_MASK_GEOMETRIC: launch_rm<RM_GEO>(p, ctas_per_sm, comp, st); break;
+    case VISS_RECON_MASK_GEOMETRIC:
+      if (comp) launch_geo<true>(p, ctas_per_sm, st);
+      else launch_geo<false>(p, ctas_per_sm, st);
+      break;
     default: return fail(VISS_ERR_INVALID, "unknown recon mask");
   }
   VISS_LAUNCH_CHECK("recon_fast_kernel");

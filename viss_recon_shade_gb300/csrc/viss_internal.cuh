@@ -224,8 +224,7 @@ struct PixPrepArgs {
   float4* geo;    // {unit s, j bits}
   int2* qr;       // {i / res, i % res} of the fine index i the REF windows test
   const int32_t* widx;  // i = widx[j] (NULL: i = j)
-  float4* bcaps;        // recon, geometric: caps of the pixel blocks and of the warps' patches (or NULL)
-  float4* wcaps;
+  float4* wcaps;        // recon, geometric: caps of the warps' patches (or NULL)
 };
 
 // Satellites of a geometric pass: directions and, for the reconstruction, snapshot cones.
@@ -250,7 +249,8 @@ struct ChannelRows {
 // Row records (both passes):
 //   rows0 {U, V, W, bias}            integer uvw and the fixed-point phase bias
 //   rows1 {f_u, f_v, f_w, c}         fractional uvw; c = |wgt V| (recon) or 0 (vis)
-//   rowsat packed satellite indices  (geometric mask)
+//   rowsat packed satellite indices  (geometric mask, vis)
+//   rowpm  {snapshot, the two satellites as bits of its satellites}  (geometric mask, recon)
 //   rowsf {U, V, W as float, 0}      (compensation)
 //   win                              vis REF: {lo_a, lo_b, M1, M2}; recon REF: {tmax, pmax, 0, 0}
 struct RowPrepArgs {
@@ -275,6 +275,7 @@ struct RowPrepArgs {
   int4* rows0;
   float4* rows1;
   int* rowsat;
+  int2* rowpm;
   float4* uf;
   int4* win;
   int* flags;   // [0] |= any fractional uvw, [1] |= |U| out of range, |= 2 bad satellite index
@@ -349,13 +350,12 @@ struct ReconParams {
   const int2* pqr;
   const int4* rows0;
   const float4* rows1;
-  const int* rowsat;
+  const int2* rowpm;
   const float4* rowsf;
   const int4* win;
   const float4* satdir;
   const float4* scones;   // [S*2] per-snapshot cones
-  const float4* bcones;   // [npb*2] bounding cone of each pixel block: {axis, cos r}, {sin r}
-  const float4* wcones;   // [npb*2*REC_THREADS/32] the same per warp's patch of 32*REC_TJ positions
+  const float4* wcones;   // [npb*2*REC_THREADS/32] cap of each patch of 32*REC_TJ positions: {axis, cos r}, {sin r}
   const float* l;
   const float* m;
   const float* n;
@@ -369,7 +369,7 @@ struct ReconParams {
   int nsat;
   double R;
   int recon_mask;
-  // work items (segment, pixel block): segments are row ranges of one channel,
+  // work items (segment, pixel block; geometric: patch): segments are row ranges of one channel,
   // longest first; item i is segment i / npb, pixel block i % npb
   int nitems;
   int npb;
@@ -377,7 +377,7 @@ struct ReconParams {
   int64_t seg_lo[VISS_MAX_SEG], seg_hi[VISS_MAX_SEG];
   int seg_ch[VISS_MAX_SEG], seg_slot[VISS_MAX_SEG];   // slot -1: the segment writes F directly
   float ch_norm[VISS_MAX_CH];
-  int row_tile;           // visibility rows per tile: 0 REC_Q, 1 REC_Q / 2, 2 2 * REC_Q (geometric, not compensated: 4 * REC_Q)
+  int row_tile;           // visibility rows per tile: 0 REC_Q, 1 REC_Q / 2, 2 2 * REC_Q (unmasked and REF)
 };
 
 // Per-channel sum of partial slots (channels split into several segments).
