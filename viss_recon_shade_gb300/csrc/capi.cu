@@ -1,5 +1,6 @@
 // capi.cu -- the extern "C" entry points of libvissgb.so for the DFT passes:
 // argument checks, workspace layout, launch planning and kernel dispatch.
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <string>
@@ -238,7 +239,7 @@ struct RecPlan {
 
 // Recon work: every channel's rows cut into segments of about L rows, L chosen
 // for ~rec_items work items (segment x pixel block) per resident CTA; at most
-// VISS_MAX_SEG segments.  Segments are ordered longest first.
+// VISS_MAX_SEG segments, ordered longest first.
 static void plan_segments(RecPlan& p, const viss_dft_cfg& cfg, const Batch& bt, const Tuning& tn) {
   int64_t unit = REC_Q;
   const int nch = bt.ch.nch;
@@ -248,7 +249,7 @@ static void plan_segments(RecPlan& p, const viss_dft_cfg& cfg, const Batch& bt, 
   int64_t L = p.npb > 0 ? (p.K * p.npb + target - 1) / target : p.K;
   // A small pass has fewer than 4 segments of REC_Q rows per CTA: shorter ones, down to
   // REC_MIN_ROWS, so that every SM has work.  3,360 rows x 2,048 pixels: 58 -> 20 us;
-  // 28,672 x 12,288: REF windows 256 rows 190 us, 128 rows 184 us, geometric 252 us either way.
+  // 28,672 x 12,288: REF windows 256 rows 190 us, 128 rows 184 us.
   if (tn.rec_items <= 0 && L < unit) {
     while (unit > REC_MIN_ROWS && p.K * p.npb < 4 * (target / 64) * unit) unit >>= 1;
     L = unit;
@@ -263,6 +264,17 @@ static void plan_segments(RecPlan& p, const viss_dft_cfg& cfg, const Batch& bt, 
     return n;
   };
   while (count(L) > VISS_MAX_SEG) L = round_up(L + (L > 256 ? L / 4 : 0) + 1, unit);
+  // With four items per CTA or more, segment i of a channel's n holds rows up to
+  // 1.8 x - 0.8 x^2 of them (x = i / n): from 1.8 of the mean down to 0.2.  Taken longest first,
+  // the short ones level the last wave, which equal ones leave up to half empty (the number
+  // of segments is bounded by VISS_MAX_SEG, so a tall narrow pass has long ones).  Geometric
+  // 28,672 x 12,288 210 -> 197 us, 229,376 x 12,288 1581 -> 1475 us, 458,752 x 49,152 10.47 -> 10.20 ms,
+  // 1,835,008 x 196,608 150.0 -> 148.4 ms; REF windows 28,672 x 12,321 187.7 -> 183.1 us; 1.9 x - 0.9 x^2
+  // is the same within 0.3 %.  Fewer items than that all start at once, and the longest decides:
+  // 3,360 x 2,048 17.6 -> 23.1 us, so there they stay equal.
+  const int64_t ctas = planned_ctas(tn, rec_ctas(cfg.recon_mask, p.comp));
+  const int64_t g = count(L) * p.npb >= 4 * ctas ? 8 : 0;
+  auto bound = [g](int64_t kc, int64_t i, int64_t n) { return kc * ((10 + g) * i * n - g * i * i) / (10 * n * n); };
   struct Seg { int64_t lo, hi; int ch, idx; };
   Seg segs[VISS_MAX_SEG];
   int ns = 0, slots = 0;
@@ -272,18 +284,13 @@ static void plan_segments(RecPlan& p, const viss_dft_cfg& cfg, const Batch& bt, 
     p.slot0[c] = slots;
     p.nslot_ch[c] = n > 1 ? (int)n : 0;
     for (int64_t i = 0; i < n; ++i) {
-      segs[ns] = Seg{r0 + kc * i / n, r0 + kc * (i + 1) / n, c, n > 1 ? slots + (int)i : -1};
+      segs[ns] = Seg{r0 + bound(kc, i, n), r0 + bound(kc, i + 1, n), c, n > 1 ? slots + (int)i : -1};
       ++ns;
     }
     if (n > 1) slots += (int)n;
   }
   // longest first (stable)
-  for (int i = 1; i < ns; ++i) {
-    const Seg s = segs[i];
-    int j = i - 1;
-    while (j >= 0 && segs[j].hi - segs[j].lo < s.hi - s.lo) { segs[j + 1] = segs[j]; --j; }
-    segs[j + 1] = s;
-  }
+  std::stable_sort(segs, segs + ns, [](const Seg& a, const Seg& b) { return a.hi - a.lo > b.hi - b.lo; });
   p.nseg = ns;
   p.nslot = slots;
   for (int i = 0; i < ns; ++i) {
