@@ -160,7 +160,7 @@ static void plan_vis(VisPlan& p, const viss_dft_cfg& cfg, const Batch& bt, int64
   // sky chunk) per resident CTA: blocks see different occluded fractions of the sky,
   // and short items balance them (10 MHz vis: 1 chunk 158 ms, 2 149 ms, 9 143.3 ms,
   // 16 142.6 ms, 24 142.5 ms).
-  const int64_t slots = planned_ctas(tn, VISS_VIS_MINB);
+  const int64_t slots = planned_ctas(tn, vis_ctas(cfg.mask_mode, p.comp));
   int64_t nsplit = 1;
   if (tn.vis_split > 0) nsplit = tn.vis_split;
   else if (p.nrb > 0 && p.nrb < 64 * slots) nsplit = (64 * slots + p.nrb - 1) / p.nrb;
@@ -172,10 +172,12 @@ static void plan_vis(VisPlan& p, const viss_dft_cfg& cfg, const Batch& bt, int64
   // VIS_MIN_CHUNK, so that every SM has work and the last wave is short (a power of two,
   // so that a chunk stays within the VIS_P positions one REF range entry covers).  3,360 rows x
   // 2,048 pixels: 93 -> 24 us; 28,672 x 12,288: geometric 197 (512 pixels), 185 (256), 206
-  // (128) us, REF windows 184 / 170 / 169 us.
+  // (128) us, REF windows 184 / 170 / 169 us.  The unmasked instance with its fourth CTA: 4 chunks
+  // (28,672 x 12,288: 2 chunks 186 us, 3 179, 4 171.5; with three CTAs it took 175.6).
   if (tn.vis_split <= 0) {
     int64_t chunk = VIS_P;
-    while (chunk > VIS_MIN_CHUNK && p.nrb * ((J + chunk - 1) / chunk) < 2 * slots) chunk >>= 1;
+    while (chunk > VIS_MIN_CHUNK && p.nrb * ((J + chunk - 1) / chunk) < (vis_ctas(cfg.mask_mode, p.comp) > VISS_VIS_MINB ? 4 : 2) * slots)
+      chunk >>= 1;
     if (chunk < VIS_P) p.jchunk = chunk;
   }
   if (p.jchunk <= 0) p.jchunk = VIS_P;

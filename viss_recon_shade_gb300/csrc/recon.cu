@@ -25,6 +25,7 @@
 // reduced in a fixed order.
 #include <type_traits>
 
+#include "terms.cuh"
 #include "viss_internal.cuh"
 
 namespace viss {
@@ -49,98 +50,6 @@ __device__ __forceinline__ void rec_term(const int4& r0, const float4& r1, const
   __sincosf(x, &sn, &cs);
   fr = fmaf(c, cs, fr);
   fi = fmaf(c, sn, fi);
-}
-
-// Two FP32 values in one 64-bit register pair; sm_103a's packed operations round each half as
-// the single ones do.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float a, float b) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
-
-// sin and cos of two angles (half a turn added), weighted into packed sums.
-__device__ __forceinline__ void sincos2(f32x2 x, f32x2 c, f32x2& fr, f32x2& fi) {
-  float xa, xb, sa, ca, sb, cb;
-  unpack2(x, xa, xb);
-  __sincosf(xa, &sa, &ca);
-  __sincosf(xb, &sb, &cb);
-  fr = fma2(c, pack2(ca, cb), fr);
-  fi = fma2(c, pack2(sa, sb), fi);
-}
-
-// Two terms without the SFU, for phases that are all fixed point (integer uvw): the top bit of
-// the phase (shifted by a quarter turn) is the sign of the term, the next 23 bits the
-// angle r in half turns, |r| <= 1/2, and sin(pi r) and cos(pi r) are polynomials in r^2 (least
-// maximum error by iteratively reweighted least squares; in FP32 they are off by 6e-8 rms,
-// the SFU's values with their angle by 2.6e-7).
-constexpr uint32_t POLY_BIAS = 128u + 0xC0000000u - (uint32_t)PHASE_BIAS;  // on top of the phase bias
-__device__ __forceinline__ void poly2(uint32_t qa, uint32_t qb, f32x2 c, f32x2& fr, f32x2& fi) {
-  qa += POLY_BIAS;
-  qb += POLY_BIAS;
-  // bit 23 of q >> 8 falls on a bit that is set in 1.0f
-  const f32x2 r = add2(pack2(__uint_as_float((qa >> 8) | 0x3f800000u), __uint_as_float((qb >> 8) | 0x3f800000u)),
-                       pack2(-1.5f, -1.5f));
-  float ca, cb;
-  unpack2(c, ca, cb);
-  const f32x2 cs = pack2(__uint_as_float(__float_as_uint(ca) ^ (qa & 0x80000000u)),
-                         __uint_as_float(__float_as_uint(cb) ^ (qb & 0x80000000u)));
-  const f32x2 y = mul2(r, r);
-  f32x2 s = fma2(y, pack2(0.0772222504f, 0.0772222504f), pack2(-0.598046422f, -0.598046422f));
-  f32x2 k = fma2(y, pack2(0.219696805f, 0.219696805f), pack2(-1.33188021f, -1.33188021f));
-  s = fma2(y, s, pack2(2.55003166f, 2.55003166f));
-  k = fma2(y, k, pack2(4.05841208f, 4.05841208f));
-  s = fma2(y, s, pack2(-5.16770697f, -5.16770697f));
-  k = fma2(y, k, pack2(-4.934793f, -4.934793f));
-  s = fma2(y, s, pack2(3.1415925f, 3.1415925f));
-  k = fma2(y, k, pack2(0.99999994f, 0.99999994f));
-  fr = fma2(cs, k, fr);
-  fi = fma2(cs, mul2(r, s), fi);
-}
-
-// One visibility row's terms with two of the thread's pixels.  The row's FP32 parts stand
-// twice in shared memory ({fu, fu, fv, fv}, {fw, fw, c, c}) as packed operands.  POLY: without
-// the SFU (integer uvw only).
-template <bool FRAC, bool COMP, bool POLY>
-__device__ __forceinline__ void rec_term2(const int4& r0, const ulonglong2& fuv, f32x2 fw, const float4& rf, f32x2 c,
-                                          const int* A, const int* B, const int* C, f32x2 X, f32x2 Y, f32x2 Z, f32x2 lx,
-                                          f32x2 ly, f32x2 lz, f32x2& fr, f32x2& fi) {
-  uint32_t q[2];
-#pragma unroll
-  for (int h = 0; h < 2; ++h)
-    q[h] = (uint32_t)r0.x * (uint32_t)A[h] + (uint32_t)r0.y * (uint32_t)B[h] + (uint32_t)r0.z * (uint32_t)C[h] +
-           (uint32_t)r0.w;
-  if (POLY) {
-    poly2(q[0], q[1], c, fr, fi);
-    return;
-  }
-  f32x2 e = pack2(KM3PI, KM3PI);
-  if (FRAC) e = fma2(fuv.x, X, fma2(fuv.y, Y, fma2(fw, Z, e)));
-  if (COMP)
-    e = fma2(pack2(rf.x, rf.x), lx, fma2(pack2(rf.y, rf.y), ly, fma2(pack2(rf.z, rf.z), lz, e)));
-  const f32x2 f = pack2(__uint_as_float((q[0] >> 9) | 0x3f800000u), __uint_as_float((q[1] >> 9) | 0x3f800000u));
-  sincos2(fma2(f, pack2(K2PI, K2PI), e), c, fr, fi);
 }
 
 constexpr int RM_NONE = VISS_RECON_MASK_NONE, RM_REF = VISS_RECON_MASK_REF;
@@ -245,9 +154,9 @@ __device__ __forceinline__ void recon_rows(const ReconParams& p, RecSmem<RM, COM
       const int4 r0 = sm.r0[r];
       const ulonglong2 fuv = FRAC ? sm.r1[r] : make_ulonglong2(0ull, 0ull), fwc = sm.r2[r];
       const float4 rf = COMP ? sm.rf[r] : make_float4(0.f, 0.f, 0.f, 0.f);
-      rec_term2<FRAC, COMP, false>(r0, fuv, fwc.x, rf, fwc.y, A, B, C, XF[0], YF[0], ZF[0], LX[0], LY[0], LZ[0], tr[0],
+      term2<FRAC, COMP, false>(r0, fuv, fwc.x, rf, fwc.y, A, B, C, r0.w, r0.w, XF[0], YF[0], ZF[0], LX[0], LY[0], LZ[0], tr[0],
                                    ti[0]);
-      rec_term2<FRAC, COMP, decltype(poly)::value>(r0, fuv, fwc.x, rf, fwc.y, A + 2, B + 2, C + 2, XF[1], YF[1], ZF[1],
+      term2<FRAC, COMP, decltype(poly)::value>(r0, fuv, fwc.x, rf, fwc.y, A + 2, B + 2, C + 2, r0.w, r0.w, XF[1], YF[1], ZF[1],
                                                    LX[1], LY[1], LZ[1], tr[1], ti[1]);
     };
     if (RM == RM_REF && masked_tile) {
@@ -265,7 +174,7 @@ __device__ __forceinline__ void recon_rows(const ReconParams& p, RecSmem<RM, COM
             const int i = 2 * h + o;
             cm[o] = TP[i] >= 1 && TP[i] <= wv.x && PP[i] >= 1 && PP[i] <= wv.y ? 0.f : c;
           }
-          rec_term2<FRAC, COMP, false>(r0, fuv, fwc.x, rf, pack2(cm[0], cm[1]), A + 2 * h, B + 2 * h, C + 2 * h, XF[h],
+          term2<FRAC, COMP, false>(r0, fuv, fwc.x, rf, pack2(cm[0], cm[1]), A + 2 * h, B + 2 * h, C + 2 * h, r0.w, r0.w, XF[h],
                                        YF[h], ZF[h], LX[h], LY[h], LZ[h], tr[h], ti[h]);
         }
       }

@@ -21,6 +21,9 @@
 //   REF_*: per-row window (row range x column range on the fine grid); a warp
 //     none of whose 128 windows reaches the tile runs the unmasked loop.
 // Pixel chunks give partial sums, reduced in a fixed order.
+#include <type_traits>
+
+#include "terms.cuh"
 #include "viss_internal.cuh"
 
 namespace viss {
@@ -137,6 +140,124 @@ struct VisSmem {
   float4 acc[VIS_ROWS];           // running totals (re, im) and their Kahan compensation per visibility
   uint32_t sbits[GEO ? VIS_SAT_WORDS : 1];  // [satellite][word]: bit b = mixed pixel 32*word + b occluded
 };
+
+template <bool COMP, int P>
+struct VisSmem<VISS_MASK_NONE, COMP, P> {
+  int4 p0[P];         // {A, B, C, -}
+  ulonglong2 p1[P];   // {x, x, y, y}
+  ulonglong2 p2[P];   // {z, z, c, c}
+  float4 lo[COMP ? P : 1];
+  float4 acc[VIS_ROWS];
+};
+
+// Unmasked items.  Every FP32 operation of a term but the SFU's runs packed, two rows at a time, and
+// of integer uvw every fourth term is a polynomial (as the reconstruction's): the FMA pipe
+// has room beside the SFU there.  In 64 registers, so that a fourth CTA hides the tile
+// barriers (compensated: 80 and three).  229,376 x 49,152 fractional 5.36 -> 5.04 ms (5.41 at three
+// CTAs); 262,144 x 196,249 integer 21.8 -> 20.9 ms (20.3 at three, but the instance is the
+// same), compensated fractional 29.8 -> 27.8 ms; 200,003 x 65,537 compensated 7.60 -> 7.12 ms.  The
+// REF instances keep single terms: packed, their masked path spills (28,672 x 12,321 170 ->
+// 176 us, 262,144 x 196,249 22.2 -> 21.7 ms).
+template <bool FRAC, bool COMP, int P>
+__device__ __forceinline__ void vis_rows(const VisParams& p, VisSmem<VISS_MASK_NONE, COMP, P>& sm, int64_t rb, int split, int ch,
+                                         int64_t rb_first, int64_t row_first, int64_t nvalid) {
+  const int tid = threadIdx.x;
+  const int64_t row0 = rb * VIS_ROWS;                   // padded row of this rowblock
+  const float* bright = p.bright ? p.bright + (int64_t)ch * p.J : nullptr;
+  int U[VIS_TK], V[VIS_TK], W[VIS_TK], BI[VIS_TK];
+  // rows in packed pairs (row slot 2h in the low half, 2h + 1 in the high one)
+  f32x2 FU[VIS_TK / 2], FV[VIS_TK / 2], FW[VIS_TK / 2];
+  f32x2 UF[VIS_TK / 2], VF[VIS_TK / 2], WF[VIS_TK / 2];
+#pragma unroll
+  for (int i = 0; i < VIS_TK; ++i) {
+    const int64_t k = row0 + tid + i * VIS_THREADS;  // rows are padded to a whole block
+    const int4 r0 = p.rows0[k];
+    U[i] = r0.x; V[i] = r0.y; W[i] = r0.z; BI[i] = r0.w;
+    sm.acc[tid + i * VIS_THREADS] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (int h = 0; h < VIS_TK / 2; ++h) {
+    const int64_t k = row0 + tid + 2 * h * VIS_THREADS;
+    FU[h] = FV[h] = FW[h] = UF[h] = VF[h] = WF[h] = 0ull;
+    if (FRAC) {
+      const float4 a = p.rows1[k], b = p.rows1[k + VIS_THREADS];
+      FU[h] = pack2(a.x, b.x); FV[h] = pack2(a.y, b.y); FW[h] = pack2(a.z, b.z);
+    }
+    if (COMP) {
+      const float4 a = p.rowsf[k], b = p.rowsf[k + VIS_THREADS];
+      UF[h] = pack2(a.x, b.x); VF[h] = pack2(a.y, b.y); WF[h] = pack2(a.z, b.z);
+    }
+  }
+  const int64_t jb = (int64_t)split * p.jchunk;
+  int64_t je = jb + p.jchunk;
+  if (je > p.J) je = p.J;
+
+  for (int64_t tile = jb; tile < je; tile += P) {
+    const int np = (int)((je - tile) < P ? (je - tile) : P);
+    __syncthreads();  // previous tile fully consumed
+    for (int i = tid; i < np; i += VIS_THREADS) {
+      const int64_t j = tile + i;
+      const int4 a = p.pix0[j];
+      const float c = bright ? bright[j] : __int_as_float(a.w);
+      float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (FRAC) b = reinterpret_cast<const float4*>(p.pix1)[j];
+      sm.p0[i] = a;
+      if (FRAC) sm.p1[i] = make_ulonglong2(pack2(b.x, b.x), pack2(b.y, b.y));
+      sm.p2[i] = make_ulonglong2(pack2(b.z, b.z), pack2(c, c));
+      if (COMP) sm.lo[i] = p.plo[j];
+    }
+    __syncthreads();  // the tile's records are in shared memory
+    f32x2 tr[VIS_TK / 2], ti[VIS_TK / 2];   // this tile's sums; running totals live in sm.acc
+#pragma unroll
+    for (int h = 0; h < VIS_TK / 2; ++h) tr[h] = ti[h] = 0ull;
+    static_assert(VIS_TK == 4, "two row pairs");
+    // pixel pi with all of the thread's rows; poly: the second pair without the SFU
+    auto pixel_term = [&](int pi, auto poly) {
+      const int4 a = sm.p0[pi];
+      const ulonglong2 bxy = FRAC ? sm.p1[pi] : make_ulonglong2(0ull, 0ull), bzc = sm.p2[pi];
+      const float4 lo = COMP ? sm.lo[pi] : make_float4(0.f, 0.f, 0.f, 0.f);
+      term2<FRAC, COMP, false>(a, bxy, bzc.x, lo, bzc.y, U, V, W, BI[0], BI[1], FU[0], FV[0], FW[0], UF[0], VF[0], WF[0],
+                               tr[0], ti[0]);
+      term2<FRAC, COMP, decltype(poly)::value>(a, bxy, bzc.x, lo, bzc.y, U + 2, V + 2, W + 2, BI[2], BI[3], FU[1], FV[1],
+                                               FW[1], UF[1], VF[1], WF[1], tr[1], ti[1]);
+    };
+    int pi = 0;
+    if (!FRAC && !COMP) {
+      for (; pi + 4 <= np; pi += 4) {
+        pixel_term(pi, std::false_type{});
+        pixel_term(pi + 1, std::true_type{});
+        pixel_term(pi + 2, std::false_type{});
+        pixel_term(pi + 3, std::true_type{});
+      }
+    }
+#pragma unroll 2
+    for (; pi < np; ++pi) pixel_term(pi, std::false_type{});
+#pragma unroll
+    for (int h = 0; h < VIS_TK / 2; ++h) {
+      float r[2], im[2];
+      unpack2(tr[h], r[0], r[1]);
+      unpack2(ti[h], im[0], im[1]);
+#pragma unroll
+      for (int o = 0; o < 2; ++o) {
+        float4 t = sm.acc[tid + (2 * h + o) * VIS_THREADS];  // owned by this thread alone
+        kahan_add(t.x, t.z, r[o]);
+        kahan_add(t.y, t.w, im[o]);
+        sm.acc[tid + (2 * h + o) * VIS_THREADS] = t;
+      }
+    }
+  }
+  // V = -ar + i ai  (the angle carried an extra half turn)
+#pragma unroll
+  for (int i = 0; i < VIS_TK; ++i) {
+    const int64_t kl = (rb - rb_first) * VIS_ROWS + tid + i * VIS_THREADS;
+    const float4 t = sm.acc[tid + i * VIS_THREADS];
+    if (kl < nvalid) {
+      const int64_t k = row_first + kl;
+      if (p.nsplit == 1) p.out[k] = make_float2(-t.x, t.y);
+      else p.out[(int64_t)split * p.K + k] = make_float2(t.x, t.y);
+    }
+  }
+}
 
 template <int MASK, bool FRAC, bool COMP, int P>
 __device__ __forceinline__ void vis_body(const VisParams& p, VisSmem<MASK, COMP, P>& sm, int64_t rb, int split, int ch,
@@ -470,7 +591,7 @@ __device__ __forceinline__ void vis_body(const VisParams& p, VisSmem<MASK, COMP,
 // (channels, occluded fractions) balance without a wave tail.  The counter is
 // reset by the host before the launch; no CTA ever waits on another.
 template <int MASK, bool COMP, int P>
-__global__ void __launch_bounds__(VIS_THREADS, VISS_VIS_MINB) vis_fast_kernel(const VisParams p) {
+__global__ void __launch_bounds__(VIS_THREADS, vis_ctas(MASK, COMP)) vis_fast_kernel(const VisParams p) {
   __shared__ VisSmem<MASK, COMP, P> sm;
   __shared__ int s_item;
   const bool frac = __ldg(p.flags + FLAG_FRAC) != 0;
@@ -485,8 +606,13 @@ __global__ void __launch_bounds__(VIS_THREADS, VISS_VIS_MINB) vis_fast_kernel(co
     int ch = 0;
     while (ch + 1 < p.ch.nch && rb >= p.ch.rb_off[ch + 1]) ++ch;
     const int64_t nvalid = p.ch.row_off[ch + 1] - p.ch.row_off[ch];
-    if (frac) vis_body<MASK, true, COMP, P>(p, sm, rb, split, ch, p.ch.rb_off[ch], p.ch.row_off[ch], nvalid);
-    else vis_body<MASK, false, COMP, P>(p, sm, rb, split, ch, p.ch.rb_off[ch], p.ch.row_off[ch], nvalid);
+    if constexpr (MASK == VISS_MASK_NONE) {
+      if (frac) vis_rows<true, COMP, P>(p, sm, rb, split, ch, p.ch.rb_off[ch], p.ch.row_off[ch], nvalid);
+      else vis_rows<false, COMP, P>(p, sm, rb, split, ch, p.ch.rb_off[ch], p.ch.row_off[ch], nvalid);
+    } else {
+      if (frac) vis_body<MASK, true, COMP, P>(p, sm, rb, split, ch, p.ch.rb_off[ch], p.ch.row_off[ch], nvalid);
+      else vis_body<MASK, false, COMP, P>(p, sm, rb, split, ch, p.ch.rb_off[ch], p.ch.row_off[ch], nvalid);
+    }
   }
 }
 

@@ -86,6 +86,9 @@ constexpr int RED_GROUPS = 8;
 #define VISS_REC_MINB 3
 #endif
 
+// Resident CTAs per SM of the visibility instances (vis_dft.cu).
+constexpr int vis_ctas(int mask, bool comp) { return mask == VISS_MASK_NONE && !comp ? VISS_VIS_MINB + 1 : VISS_VIS_MINB; }
+
 // Resident CTAs per SM of the reconstruction instances (recon.cu).
 constexpr int rec_ctas(int recon_mask, bool comp) {
   return recon_mask == VISS_RECON_MASK_NONE && !comp ? VISS_REC_MINB + 1 : VISS_REC_MINB;
