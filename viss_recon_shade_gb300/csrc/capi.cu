@@ -192,7 +192,7 @@ struct RecPlan {
   int64_t seg_lo[VISS_MAX_SEG] = {}, seg_hi[VISS_MAX_SEG] = {};
   int seg_ch[VISS_MAX_SEG] = {}, seg_slot[VISS_MAX_SEG] = {};
   int slot0[VISS_MAX_CH] = {}, nslot_ch[VISS_MAX_CH] = {};
-  bool geo = false, ref = false, comp = false, plain = false, large = false;
+  bool geo = false, ref = false, comp = false, plain = false;
   int4 *pix0 = nullptr, *pix1 = nullptr, *rows0 = nullptr, *win = nullptr;
   float4 *rows1 = nullptr, *plo = nullptr, *pgeo = nullptr, *rowsf = nullptr, *satdir = nullptr, *scones = nullptr;
   float4* wcones = nullptr;
@@ -247,9 +247,7 @@ static void plan_segments(RecPlan& p, const viss_dft_cfg& cfg, const Batch& bt, 
   const int nch = bt.ch.nch;
   // items per CTA: many short segments balance blocks whose pixels the Moon hides for
   // different parts of the orbit (10 MHz recon: 4 items 191 ms, 8 176 ms, 32 167 ms, 64 165 ms)
-  p.large = p.K * p.npb >= 64 * planned_ctas(tn, rec_ctas(cfg.recon_mask, p.comp, true)) * REC_Q;
-  const int64_t ctas = planned_ctas(tn, rec_ctas(cfg.recon_mask, p.comp, p.large));
-  const int64_t target = (tn.rec_items > 0 ? tn.rec_items : 64) * ctas;
+  const int64_t target = (tn.rec_items > 0 ? tn.rec_items : 64) * planned_ctas(tn, rec_ctas(cfg.recon_mask, p.comp));
   int64_t L = p.npb > 0 ? (p.K * p.npb + target - 1) / target : p.K;
   // A small pass has fewer than 4 segments of REC_Q rows per CTA: shorter ones, down to
   // REC_MIN_ROWS, so that every SM has work.  3,360 rows x 2,048 pixels: 58 -> 20 us;
@@ -276,6 +274,7 @@ static void plan_segments(RecPlan& p, const viss_dft_cfg& cfg, const Batch& bt, 
   // 1,835,008 x 196,608 150.0 -> 148.4 ms; REF windows 28,672 x 12,321 187.7 -> 183.1 us; 1.9 x - 0.9 x^2
   // is the same within 0.3 %.  Fewer items than that all start at once, and the longest decides:
   // 3,360 x 2,048 17.6 -> 23.1 us, so there they stay equal.
+  const int64_t ctas = planned_ctas(tn, rec_ctas(cfg.recon_mask, p.comp));
   const int64_t g = count(L) * p.npb >= 4 * ctas ? 8 : 0;
   auto bound = [g](int64_t kc, int64_t i, int64_t n) { return kc * ((10 + g) * i * n - g * i * i) / (10 * n * n); };
   struct Seg { int64_t lo, hi; int ch, idx; };
@@ -571,7 +570,6 @@ int recon_impl(const viss_dft_cfg& cfg, const double scale[3], const float dlmn[
   else rp.row_tile = 2;
   rp.npb = (int)p.npb;
   rp.nseg = p.nseg;
-  rp.large = p.large;
   rp.nitems = (int)(p.nseg * p.npb);
   for (int i = 0; i < p.nseg; ++i) {
     rp.seg_lo[i] = p.seg_lo[i]; rp.seg_hi[i] = p.seg_hi[i]; rp.seg_ch[i] = p.seg_ch[i]; rp.seg_slot[i] = p.seg_slot[i];

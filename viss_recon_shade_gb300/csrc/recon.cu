@@ -403,7 +403,7 @@ __device__ __forceinline__ void recon_geo(const ReconParams& p, GeoWarp& sm, flo
 }
 
 template <bool COMP>
-__global__ void __launch_bounds__(REC_THREADS, rec_ctas(VISS_RECON_MASK_GEOMETRIC, COMP, false)) recon_geo_kernel(const ReconParams p) {
+__global__ void __launch_bounds__(REC_THREADS, rec_ctas(VISS_RECON_MASK_GEOMETRIC, COMP)) recon_geo_kernel(const ReconParams p) {
   __shared__ GeoSmem<COMP> sm;
   const bool frac = __ldg(p.flags + FLAG_FRAC) != 0;
   const int warp = threadIdx.x >> 5;
@@ -434,8 +434,8 @@ __global__ void __launch_bounds__(REC_THREADS, rec_ctas(VISS_RECON_MASK_GEOMETRI
 // the instances at their best CTAs): unmasked fractional 23.4 -> 22.3 ms, compensated 29.2 -> 27.3
 // (32.6 at four CTAs), integer with every fourth term a polynomial 21.5 -> 21.1, REF windows
 // 21.45 -> 21.26.
-template <int RM, bool COMP, int Q, bool LARGE>
-__global__ void __launch_bounds__(REC_THREADS, rec_ctas(RM, COMP, LARGE)) recon_fast_kernel(const ReconParams p) {
+template <int RM, bool COMP, int Q>
+__global__ void __launch_bounds__(REC_THREADS, rec_ctas(RM, COMP)) recon_fast_kernel(const ReconParams p) {
   __shared__ RecSmem<RM, COMP, Q> sm;
   __shared__ int s_item;
   const bool frac = __ldg(p.flags + FLAG_FRAC) != 0;
@@ -457,14 +457,8 @@ __global__ void __launch_bounds__(REC_THREADS, rec_ctas(RM, COMP, LARGE)) recon_
 
 template <int RM, bool COMP, int Q>
 static void launch_tile(const ReconParams& p, int ctas_per_sm, cudaStream_t st) {
-  constexpr bool TWO = RM == RM_REF && !COMP;
-  if (TWO && p.large) {
-    const int g = persistent_grid(recon_fast_kernel<RM, COMP, Q, TWO>, REC_THREADS, ctas_per_sm, p.nitems);
-    recon_fast_kernel<RM, COMP, Q, TWO><<<g, REC_THREADS, 0, st>>>(p);
-    return;
-  }
-  const int g = persistent_grid(recon_fast_kernel<RM, COMP, Q, false>, REC_THREADS, ctas_per_sm, p.nitems);
-  recon_fast_kernel<RM, COMP, Q, false><<<g, REC_THREADS, 0, st>>>(p);
+  const int g = persistent_grid(recon_fast_kernel<RM, COMP, Q>, REC_THREADS, ctas_per_sm, p.nitems);
+  recon_fast_kernel<RM, COMP, Q><<<g, REC_THREADS, 0, st>>>(p);
 }
 
 // Row tiles of 2 REC_Q visibilities (the default), REC_Q or REC_Q / 2 (tuning).

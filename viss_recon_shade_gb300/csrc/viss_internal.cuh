@@ -89,13 +89,9 @@ constexpr int RED_GROUPS = 8;
 // Resident CTAs per SM of the visibility instances (vis_dft.cu).
 constexpr int vis_ctas(int mask, bool comp) { return mask == VISS_MASK_NONE && !comp ? VISS_VIS_MINB + 1 : VISS_VIS_MINB; }
 
-// Resident CTAs per SM of the reconstruction instances (recon.cu).  REF windows at FAST
-// precision have one of each: fractional uvw are faster in 64 registers on a pass that fills
-// 64 items a CTA (262,144 x 196,249: three CTAs 23.9 ms, four 23.5; integer 21.4 either way),
-// smaller passes in 80 (100,000 x 12,321: 0.721 against 0.747 ms).
-constexpr int rec_ctas(int recon_mask, bool comp, bool large) {
-  return !comp && (recon_mask == VISS_RECON_MASK_NONE || (recon_mask == VISS_RECON_MASK_REF && large)) ? VISS_REC_MINB + 1
-                                                                                                     : VISS_REC_MINB;
+// Resident CTAs per SM of the reconstruction instances (recon.cu).
+constexpr int rec_ctas(int recon_mask, bool comp) {
+  return recon_mask == VISS_RECON_MASK_NONE && !comp ? VISS_REC_MINB + 1 : VISS_REC_MINB;
 }
 
 // Channels of one batched pass, and visibility segments of its reconstruction
@@ -384,7 +380,6 @@ struct ReconParams {
   int64_t seg_lo[VISS_MAX_SEG], seg_hi[VISS_MAX_SEG];
   int seg_ch[VISS_MAX_SEG], seg_slot[VISS_MAX_SEG];   // slot -1: the segment writes F directly
   float ch_norm[VISS_MAX_CH];
-  bool large;             // 64 items of REC_Q rows per CTA and more (rec_ctas)
   int row_tile;           // visibility rows per tile: 0 REC_Q, 1 REC_Q / 2, 2 2 * REC_Q (unmasked and REF)
 };
 
