@@ -96,15 +96,12 @@ __device__ __forceinline__ void recon_rows(const ReconParams& p, RecSmem<RM, COM
   // pixels in packed pairs (pixel 2h in the low half, 2h + 1 in the high one)
   f32x2 XF[REC_TJ / 2], YF[REC_TJ / 2], ZF[REC_TJ / 2];
   f32x2 LX[REC_TJ / 2], LY[REC_TJ / 2], LZ[REC_TJ / 2];
-  int TP[REC_TJ], PP[REC_TJ];
   // running totals live in sm.acc
 #pragma unroll
   for (int i = 0; i < REC_TJ; ++i) {
     const int64_t pos = j0 + i;  // pixels padded to a whole block
     const int4 a = p.pix0[pos];
     A[i] = a.x; B[i] = a.y; C[i] = a.z;
-    TP[i] = PP[i] = -1;
-    if (RM == RM_REF) { const int2 qr = p.pqr[pos]; PP[i] = qr.x; TP[i] = qr.y; }
     sm.acc[tid * REC_TJ + i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
 #pragma unroll
@@ -160,6 +157,11 @@ __device__ __forceinline__ void recon_rows(const ReconParams& p, RecSmem<RM, COM
                                                    LX[1], LY[1], LZ[1], tr[1], ti[1]);
     };
     if (RM == RM_REF && masked_tile) {
+      // the pixels' fine coordinates are read again here: held, they cost the unmasked tiles 8 of 80
+      // registers (262,144 x 196,249: integer 21.4 -> 20.9 ms, fractional 23.9 -> 23.2)
+      int TP[REC_TJ], PP[REC_TJ];
+#pragma unroll
+      for (int i = 0; i < REC_TJ; ++i) { const int2 qr = __ldg(p.pqr + j0 + i); PP[i] = qr.x; TP[i] = qr.y; }
       for (int r = 0; r < nq; ++r) {
         const int4 r0 = sm.r0[r], wv = sm.win[r];
         const ulonglong2 fuv = FRAC ? sm.r1[r] : make_ulonglong2(0ull, 0ull), fwc = sm.r2[r];
@@ -433,7 +435,7 @@ __global__ void __launch_bounds__(REC_THREADS, rec_ctas(VISS_RECON_MASK_GEOMETRI
 // 200,003 x 65,537).  Packed against single operations (262,144 x 196,249,
 // the instances at their best CTAs): unmasked fractional 23.4 -> 22.3 ms, compensated 29.2 -> 27.3
 // (32.6 at four CTAs), integer with every fourth term a polynomial 21.5 -> 21.1, REF windows
-// 21.45 -> 21.26.
+// 21.45 -> 20.9.
 template <int RM, bool COMP, int Q>
 __global__ void __launch_bounds__(REC_THREADS, rec_ctas(RM, COMP)) recon_fast_kernel(const ReconParams p) {
   __shared__ RecSmem<RM, COMP, Q> sm;
