@@ -16,7 +16,8 @@
 //     no per-term test) and a mixed list.  Each (mixed pixel, satellite of the
 //     block's rows) pair is decided once per tile into shared-memory bits (in
 //     double within GEO_EPS of the limb); a term ORs its row's two satellite
-//     bits.  Blocks whose rows span too many satellites for the bits test the
+//     bits, after the warp has dropped the mixed pixels hidden from all its rows and
+//     run those hidden from none without a test.  Blocks whose rows span too many satellites for the bits test the
 //     row's two satellites per term instead.
 //   REF_*: per-row window (row range x column range on the fine grid); a warp
 //     none of whose 128 windows reaches the tile runs the unmasked loop.
