@@ -137,8 +137,12 @@ __device__ void prep_pixels_caps(const PixPrepArgs& a, int block, float4* wcaps)
   const float4 wa = cap_axis(sx, sy, sz);
   float c2 = 0.f;
 #pragma unroll
-  for (int i = 0; i < REC_TJ; ++i)
-    if (p0 + 32 * i < a.J) c2 = fmaxf(c2, chord2(wa, g[i]));
+  for (int i = 0; i < REC_TJ; ++i) {
+    // no direction (0, 0, 0), which no satellite hides: a cap of 90 degrees, which no snapshot hides
+    // as a whole (half angles of shadows are below that).  Its chord, 1, would pass for 60 degrees.
+    const bool none = g[i].x == 0.f && g[i].y == 0.f && g[i].z == 0.f;
+    if (p0 + 32 * i < a.J) c2 = fmaxf(c2, none ? 2.f : chord2(wa, g[i]));
+  }
   c2 = warp_max(c2);
   if (lane == 0) cap_write(wa, c2, wcaps + 2 * ((int64_t)block * (REC_THREADS / 32) + warp));
 }
