@@ -502,6 +502,7 @@ int launch_recon_fast(const ReconParams& p, int ctas_per_sm, bool comp, cudaStre
 // (s + e) * f, rounded once (but for the last bits of e)
 __device__ __forceinline__ float pair_times(const FloatPair& v, float f) {
   const float h = __fmul_rn(v.s, f);
+  if (isinf(h)) return h;
   return h + __fmaf_rn(v.e, f, __fmaf_rn(v.s, f, -h));
 }
 
@@ -512,10 +513,17 @@ __global__ void __launch_bounds__(32 * RED_GROUPS) recon_reduce_kernel(const Rec
   const int c = blockIdx.y;
   if (p.nslot[c] == 0) return;
   FloatPair re, im;
-  reduce_partials(p.partial + (int64_t)p.slot0[c] * p.J + pos, p.nslot[c], p.J, pos < p.J, re, im);
+  const float2* const part = p.partial + (int64_t)p.slot0[c] * p.J + pos;
+  const float norm = p.norm[c];
+  reduce_partials(part, p.nslot[c], p.J, pos < p.J, re, im);
   if (threadIdx.x < 32 && pos < p.J) {
     const int64_t j = p.perm ? (int64_t)p.perm[pos] : pos;
-    p.out[(int64_t)c * p.J + j] = make_float2(pair_times(re, -p.norm[c]), pair_times(im, -p.norm[c]));
+    float2 o = make_float2(pair_times(re, -norm), pair_times(im, -norm));
+    if (!re.in_range() || !im.in_range()) {
+      const double2 d = sum_partials_f64(part, p.nslot[c], p.J);
+      o = make_float2((float)(-d.x * norm), (float)(-d.y * norm));
+    }
+    p.out[(int64_t)c * p.J + j] = o;
   }
 }
 

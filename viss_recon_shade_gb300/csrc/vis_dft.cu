@@ -656,7 +656,14 @@ __global__ void __launch_bounds__(32 * RED_GROUPS) vis_reduce_kernel(const float
   const int64_t k = (int64_t)blockIdx.x * 32 + (threadIdx.x & 31);
   FloatPair re, im;
   reduce_partials(part + k, nsplit, K, k < K, re, im);
-  if (threadIdx.x < 32 && k < K) out[k] = make_float2(-(re.s + re.e), im.s + im.e);
+  if (threadIdx.x < 32 && k < K) {
+    float2 o = make_float2(-(re.s + re.e), im.s + im.e);
+    if (!re.in_range() || !im.in_range()) {
+      const double2 d = sum_partials_f64(part + k, nsplit, K);
+      o = make_float2((float)-d.x, (float)d.y);
+    }
+    out[k] = o;
+  }
 }
 
 int launch_vis_reduce(const float2* partial, int nsplit, int64_t K, float2* out, cudaStream_t st) {

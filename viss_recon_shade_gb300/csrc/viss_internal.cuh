@@ -169,12 +169,27 @@ struct FloatPair {
     e = __fadd_rn(e, __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(x, b)));
     s = t;
   }
+  // false once an addend or a sum on the way was out of FP32's range (s and e stay infinite or NaN)
+  __device__ __forceinline__ bool in_range() const { return fabsf(s) <= 3.402823466e38f && fabsf(e) <= 3.402823466e38f; }
 };
+
+// The same sum in double, one addend after another: for pairs that left FP32's range, where the sum
+// may be finite all the same, or infinite and not NaN.
+static __device__ __noinline__ double2 sum_partials_f64(const float2* part, int n, int64_t stride) {
+  double2 r = make_double2(0.0, 0.0);
+  for (int s = 0; s < n; ++s) {
+    const float2 v = part[(int64_t)s * stride];
+    r.x += v.x;
+    r.y += v.y;
+  }
+  return r;
+}
 
 // The sum over s < n of part[s * stride] (s in a fixed order: this warp's every RED_GROUPS-th,
 // then the warps' sums in order); valid in warp 0.  Float pairs, not double: at 2 FP64 lanes
 // per SM and clock the conversions and additions of double sums took five times the HBM reads
 // of the partials (10 MHz vis: 31M partials, 266 us).  Four loads are in flight per thread.
+// The caller takes sum_partials_f64 where a pair is not in_range.
 __device__ __forceinline__ void reduce_partials(const float2* part, int n, int64_t stride, bool live, FloatPair& re,
                                                 FloatPair& im) {
   __shared__ float4 sums[RED_GROUPS][32];
