@@ -957,8 +957,9 @@ static int imagerecon_impl(int uvw_index, int lmnC_index, int res, float* F, con
   const float* ratios[4] = {thetaP0, phiP0, dtheta, dphi};
   rc = recon_impl(cfg, scale, dlmn, sky, vis, bt, nullptr, Tuning{}, viss, F, ws, p.bytes, st,
                   masked ? ratios : nullptr);
-  if (rc == VISS_OK && masked && !plain_precision(precision)) {
-    // rows whose ratio arrays are not of the reference's form are rejected
+  if (rc == VISS_OK && masked && !plain_precision(precision) && uvw_index > 0 && lmnC_index > 0) {
+    // rows whose ratio arrays are not of the reference's form are rejected (an empty pass returns
+    // before it clears the flag words)
     int flags[2] = {0, 0};
     p.layout(ws);
     cudaError_t e = cudaMemcpyAsync(flags, p.flags, sizeof(flags), cudaMemcpyDeviceToHost, st);
