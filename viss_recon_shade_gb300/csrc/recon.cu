@@ -84,7 +84,7 @@ __device__ __forceinline__ void recon_store(const ReconParams& p, const float4* 
 }
 
 // Unmasked and REF-mask items.  Every FP32 operation of a term but the SFU's runs packed, two pixels
-// at a time, and of integer uvw every fourth term is a polynomial: the FMA pipe has room
+// at a time, and of integer uvw a quarter of the terms are polynomials: the FMA pipe has room
 // beside the SFU there (10 of its 16 cycles a warp-term).  What it measured against single
 // operations is at recon_fast_kernel.
 template <int RM, bool FRAC, bool COMP, int Q>
@@ -183,10 +183,14 @@ __device__ __forceinline__ void recon_rows(const ReconParams& p, RecSmem<RM, COM
     } else {
       int r = 0;
       if (!FRAC && !COMP) {
+        // the polynomial in two adjacent rows of four: the records alternate the sign of |y| so that
+        // the SFU's systematic error cancels over the rows, which needs both signs in each kind of term
+        // (in every other row: |mean error| of those pixels 9e-9 against 1e-10 at 65,536 rows).
+        // Rows with and without it in turn: 262,144 x 196,249 in row order 2 % slower.
         for (; r + 4 <= nq; r += 4) {
           row_term(r, std::false_type{});
-          row_term(r + 1, std::true_type{});
-          row_term(r + 2, std::false_type{});
+          row_term(r + 2, std::true_type{});
+          row_term(r + 1, std::false_type{});
           row_term(r + 3, std::true_type{});
         }
       }
