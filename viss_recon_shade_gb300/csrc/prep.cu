@@ -309,14 +309,17 @@ __device__ __forceinline__ float4 sat_direction(const float* pos, double R) {
 // from every one.  cone[0] = {c, cos_occ}, cone[1] = {cos_vis, sin_occ, sin_vis, -}
 // (the sines of the two angles, 0 where the cosine is the 2 / -2 of "never").
 // Degenerate sets (a satellite at the origin) get cos_occ = 2, cos_vis = -2.
-// In FP32: rho from the largest chord, alpha from the extreme cosines; each is good to 3e-7
-// rad, which the margins (1.2e-5 rad, 1.5e-6 in the cosine tested against) cover many times over.
+// In FP32: rho from the largest chord, good to 3e-7 rad, which the margins (1.2e-5 rad, 1.5e-6 in the
+// cosine tested against) cover many times over; alpha from the extreme cosines, which are good to
+// 6e-8 only and leave alpha itself uncertain by 6e-8 / sin(alpha) (6e-5 rad for a satellite a thousand
+// radii away), so they are widened by that first.
+constexpr float COS_ERR = 1.2e-7f;
 __device__ void cone_write(const float4& axis, float c2, float wmin, float wmax, bool degen, float4* out) {
   const float eps = 1.2e-5f;
   float cos_occ = 2.f, cos_vis = -2.f, sin_occ = 0.f, sin_vis = 0.f;
   if (!degen) {
     const float rho = 2.f * asinf(fminf(1.f, 0.5f * sqrtf(c2)));
-    const float lo = acosf(fminf(1.f, wmax)) - rho - eps, hi = acosf(fmaxf(-1.f, wmin)) + rho + eps;
+    const float lo = acosf(fminf(1.f, wmax + COS_ERR)) - rho - eps, hi = acosf(wmin - COS_ERR) + rho + eps;
     if (lo > 0.f) { cos_occ = cosf(lo) + 1.5e-6f; sin_occ = sinf(lo); }
     if (hi < 3.1415926f) { cos_vis = cosf(hi) - 1.5e-6f; sin_vis = sinf(hi); }
   }
