@@ -489,9 +489,9 @@ __device__ __forceinline__ void dedup_insert(uint64_t* tkeys, uint32_t* tidx, ui
 // The same for rows that mostly bring a new key or one last seen long ago (the
 // fused pass): the row index is lowered by a reduction that does not wait for
 // its result, one dependent trip fewer per insert.
-__device__ __forceinline__ void dedup_insert_red(uint64_t* tkeys, uint32_t* tidx, uint64_t mask, uint64_t key,
+__device__ __forceinline__ void dedup_insert_red(uint64_t* tkeys, uint32_t* tidx, uint32_t mask, uint64_t key,
                                                  uint32_t k, int* overflow) {
-  uint64_t h = dedup_hash(key) & mask;
+  uint32_t h = (uint32_t)dedup_hash(key) & mask;
   for (int probe = 0; probe < DEDUP_PROBES; ++probe, h = (h + 1) & mask) {
     uint64_t cur = *((volatile uint64_t*)(tkeys + h));
     if (cur == DEDUP_EMPTY) {
@@ -512,6 +512,15 @@ __global__ void dedup_hash_kernel(const float* u, const float* v, const float* w
   if (k >= K) return;
   dedup_insert(tkeys, tidx, mask, uvw_key(u[k], v[k], w[k], bad), (uint32_t)k, overflow);
 }
+
+// Device counters of a table pass, read back in one copy.
+struct DedupCounters {
+  int bad, overflow;  // keys out of range; a key found no slot
+  int maxdev;         // largest |coordinate| among the unique keys
+  uint32_t slots;     // the table's size (unique pass)
+  int64_t n;          // unique keys
+  unsigned long long changes;  // sampled rows whose key differs from the snapshot's before (unique pass)
+};
 
 // Fused baselines + hash pass over the rows (snapshot g, pair q) of float
 // positions [S][nsat][3], ranked pair-major (row q * S + g) as the reference
@@ -578,17 +587,78 @@ __device__ __forceinline__ void row_keys(const float* d, double lambda, float2 s
   *kr = ((uint64_t)fr[0] << 42) | ((uint64_t)fr[1] << 21) | (uint64_t)fr[2];
 }
 
+// How many rows will be inserted: the rows whose key differs from their snapshot's before, counted over
+// SAMPLE_STEPS of every SAMPLE_STRIDE snapshots.  They bound the unique rows, closely for an orbit, where a
+// key seldom comes back (403,200 snapshots of 8 satellites: 1.27 of them at 1 MHz, 1.02 at 30 MHz).
+constexpr int SAMPLE_STEPS = 4, SAMPLE_STRIDE = 256;
+
+__global__ void __launch_bounds__(256) unique_sample_kernel(const float* __restrict__ pos, int64_t S, int nsat, int ordered,
+                                                            double lambda, float2 scale, DedupCounters* cnt) {
+  const int nup = nsat * (nsat - 1) / 2;
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t chunk = t / nup, g0 = chunk * SAMPLE_STRIDE;
+  int changes = 0;
+  if (g0 + 1 < S) {
+    int m, n;
+    pair_of((int)(t - chunk * nup), nsat, 0, &m, &n);
+    uint64_t prevf = 0, prevr = 0;
+    float d[SAMPLE_STEPS + 1][3];
+#pragma unroll
+    for (int j = 0; j <= SAMPLE_STEPS; ++j) {
+      const int64_t g = g0 + j < S ? g0 + j : S - 1;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) d[j][c] = __ldg(pos + (g * nsat + n) * 3 + c) - __ldg(pos + (g * nsat + m) * 3 + c);
+    }
+#pragma unroll
+    for (int j = 0; j <= SAMPLE_STEPS; ++j) {
+      uint64_t kf, kr = 0;
+      bool oor = false;
+      row_keys(d[j], lambda, scale, ordered, &kf, &kr, &oor);
+      if (j > 0 && g0 + j < S) changes += (kf != prevf) + (ordered && kr != prevr);
+      prevf = kf;
+      prevr = kr;
+    }
+  }
+  changes = __reduce_add_sync(0xffffffffu, changes);
+  if ((threadIdx.x & 31) == 0 && changes) atomicAdd(&cnt->changes, (unsigned long long)changes);
+}
+
+// Sampled steps of one satellite pair.
+static int64_t sampled_steps(int64_t S) {
+  const int64_t whole = (S - 1) / SAMPLE_STRIDE, rest = (S - 1) % SAMPLE_STRIDE;
+  return whole * SAMPLE_STEPS + (rest < SAMPLE_STEPS ? rest : SAMPLE_STEPS);
+}
+
+// The table's size, half full with the rows expected of the sample (lo to hi slots), and the empty table.
+__global__ void __launch_bounds__(256) unique_table_kernel(uint64_t* tkeys, uint32_t* tidx, int64_t S, int npairs, int64_t steps,
+                                                           uint32_t lo, uint32_t hi, DedupCounters* cnt) {
+  uint32_t T = lo;
+  if (lo < hi) {
+    const int64_t rows = (int64_t)cnt->changes * (S - 1) / steps + npairs;
+    while (T < hi && (int64_t)T < 2 * rows) T <<= 1;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) cnt->slots = T;
+  const ulonglong2 none = make_ulonglong2(DEDUP_EMPTY, DEDUP_EMPTY);
+  for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < T / 4; i += gridDim.x * 256) {
+    reinterpret_cast<ulonglong2*>(tkeys)[2 * i] = none;
+    reinterpret_cast<ulonglong2*>(tkeys)[2 * i + 1] = none;
+    reinterpret_cast<uint4*>(tidx)[i] = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
+  }
+}
+
 __global__ void __launch_bounds__(256, UNIQUE_CTAS) unique_insert_kernel(const float* __restrict__ pos, int64_t S, int nsat,
                                                             int ordered, int run, double lambda, float2 scale,
-                                                            uint64_t* tkeys, uint32_t* tidx, uint64_t mask, int* bad,
-                                                            int* overflow) {
+                                                            uint64_t* tkeys, uint32_t* tidx, DedupCounters* cnt) {
+  int* const overflow = &cnt->overflow;
+  if (*(volatile int*)overflow) return;  // the pass is repeated with a larger table
+  const uint32_t mask = cnt->slots - 1;
   const int nup = nsat * (nsat - 1) / 2;  // satellite pairs m < n
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t chunk = t / nup;
   const int up = (int)(t - chunk * nup);
   const int64_t g0 = chunk * run;
   if (g0 >= S) return;
-  const int cnt = (int)(g0 + run < S ? run : S - g0);
+  const int steps = (int)(g0 + run < S ? run : S - g0);
   int m, n;
   pair_of(up, nsat, 0, &m, &n);
   // row offsets within a snapshot: (m, n) and, ordered, (n, m) (pair_of's order)
@@ -597,7 +667,7 @@ __global__ void __launch_bounds__(256, UNIQUE_CTAS) unique_insert_kernel(const f
   const int stride = nsat * 3;
   const float* pm = pos + (g0 * nsat + m) * 3;
   const float* pn = pos + (g0 * nsat + n) * 3;
-  const float* pend = pos + (g0 + cnt) * nsat * 3;  // prefetches stay inside the chunk
+  const float* pend = pos + (g0 + steps) * nsat * 3;  // prefetches stay inside the chunk
   // keys of the snapshot before the chunk: a row equal to it is no first occurrence
   uint64_t prevf = DEDUP_EMPTY, prevr = DEDUP_EMPTY;  // no key equals it (bit 63 is never set)
   bool oor = false;
@@ -611,19 +681,19 @@ __global__ void __launch_bounds__(256, UNIQUE_CTAS) unique_insert_kernel(const f
   // 6 CTAs per SM (40 registers; 4 CTAs without spills measured 11% slower): a
   // batch of 4 spilled ~1.5x as much and took 10.2 ms on the MIncline campaign
   // against 9.8 ms for 1 or 2.
-  for (int j0 = 0; j0 < cnt; j0 += UNIQUE_BATCH) {
+  for (int j0 = 0; j0 < steps; j0 += UNIQUE_BATCH) {
     const float* ahead = pn + (j0 + 32) * stride;
     if (ahead < pend) asm volatile("prefetch.global.L2 [%0];" ::"l"(ahead));
     float d[UNIQUE_BATCH][3];
 #pragma unroll
     for (int j = 0; j < UNIQUE_BATCH; ++j) {
-      const int o = (j0 + j < cnt ? j0 + j : cnt - 1) * stride;
+      const int o = (j0 + j < steps ? j0 + j : steps - 1) * stride;
 #pragma unroll
       for (int c = 0; c < 3; ++c) d[j][c] = __ldg(pn + o + c) - __ldg(pm + o + c);
     }
 #pragma unroll
     for (int j = 0; j < UNIQUE_BATCH; ++j) {
-      if (j0 + j >= cnt) break;
+      if (j0 + j >= steps) break;
       uint64_t kf, kr;
       row_keys(d[j], lambda, scale, ordered, &kf, &kr, &oor);
       if (kf != prevf) dedup_insert_red(tkeys, tidx, mask, kf, rowf, overflow);
@@ -636,61 +706,66 @@ __global__ void __launch_bounds__(256, UNIQUE_CTAS) unique_insert_kernel(const f
       }
     }
   }
-  if (oor) atomicOr(bad, 1);
+  if (oor) atomicOr(&cnt->bad, 1);
 }
 
 // occupied slots -> (key, first row) pairs, in any order (they are sorted next).
-// A block takes COMPACT_SLOTS slots and one atomic on the counter.
+// A block takes COMPACT_SLOTS slots at a time and one atomic on the counter.  T = 0: the size the pass
+// chose.  Nothing after an overflow, when the pass is repeated.
 constexpr int COMPACT_PER_THREAD = 16;
 constexpr int COMPACT_SLOTS = 256 * COMPACT_PER_THREAD;
 
-__global__ void __launch_bounds__(256) unique_compact_kernel(const uint64_t* tkeys, const uint32_t* tidx, int64_t T,
-                                                             uint64_t* k1, uint32_t* i1,
-                                                             unsigned long long* count, int* maxdev) {
+__global__ void __launch_bounds__(256, 4) unique_compact_kernel(const uint64_t* tkeys, const uint32_t* tidx, int64_t T,
+                                                             uint64_t* k1, uint32_t* i1, DedupCounters* cnt) {
   __shared__ unsigned warp_sum[8];
   __shared__ unsigned long long block_base;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int64_t base = (int64_t)blockIdx.x * COMPACT_SLOTS + tid;
-  uint64_t keys[COMPACT_PER_THREAD];
-  unsigned mine = 0;
+  if (cnt->overflow) return;
+  if (T == 0) T = cnt->slots;
   int dev = 0;  // largest |coordinate| of this thread's keys
+  for (int64_t tile = blockIdx.x; tile * COMPACT_SLOTS < T; tile += gridDim.x) {
+    const int64_t base = tile * COMPACT_SLOTS + tid;
+    uint64_t keys[COMPACT_PER_THREAD];
+    unsigned mine = 0;
 #pragma unroll
-  for (int i = 0; i < COMPACT_PER_THREAD; ++i) {
-    const int64_t sl = base + (int64_t)i * 256;
-    keys[i] = sl < T ? tkeys[sl] : DEDUP_EMPTY;
-    if (keys[i] != DEDUP_EMPTY) {
-      ++mine;
+    for (int i = 0; i < COMPACT_PER_THREAD; ++i) {
+      const int64_t sl = base + (int64_t)i * 256;
+      keys[i] = sl < T ? tkeys[sl] : DEDUP_EMPTY;
+      if (keys[i] != DEDUP_EMPTY) {
+        ++mine;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) dev = max(dev, abs((int)((keys[i] >> (21 * c)) & 0x1fffff) - 1048576));
+        for (int c = 0; c < 3; ++c) dev = max(dev, abs((int)((keys[i] >> (21 * c)) & 0x1fffff) - 1048576));
+      }
+    }
+    unsigned incl = mine;  // inclusive warp scan
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    __syncthreads();  // the last tile's sums are read
+    if (lane == 31) warp_sum[wid] = incl;
+    __syncthreads();
+    unsigned before = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      before += w < wid ? warp_sum[w] : 0;
+      total += warp_sum[w];
+    }
+    if (tid == 0) block_base = total ? atomicAdd((unsigned long long*)&cnt->n, (unsigned long long)total) : 0ull;
+    __syncthreads();
+    unsigned long long at = block_base + before + incl - mine;
+#pragma unroll
+    for (int i = 0; i < COMPACT_PER_THREAD; ++i) {
+      if (keys[i] != DEDUP_EMPTY) {
+        k1[at] = keys[i];
+        i1[at] = tidx[base + (int64_t)i * 256];
+        ++at;
+      }
     }
   }
   dev = __reduce_max_sync(0xffffffffu, dev);
-  if (lane == 0 && dev > 0) atomicMax(maxdev, dev);
-  unsigned incl = mine;  // inclusive warp scan
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
-  }
-  if (lane == 31) warp_sum[wid] = incl;
-  __syncthreads();
-  unsigned before = 0, total = 0;
-#pragma unroll
-  for (int w = 0; w < 8; ++w) {
-    before += w < wid ? warp_sum[w] : 0;
-    total += warp_sum[w];
-  }
-  if (tid == 0) block_base = total ? atomicAdd(count, (unsigned long long)total) : 0ull;
-  __syncthreads();
-  unsigned long long at = block_base + before + incl - mine;
-#pragma unroll
-  for (int i = 0; i < COMPACT_PER_THREAD; ++i) {
-    if (keys[i] != DEDUP_EMPTY) {
-      k1[at] = keys[i];
-      i1[at] = tidx[base + (int64_t)i * 256];
-      ++at;
-    }
-  }
+  if (lane == 0 && dev > 0) atomicMax(&cnt->maxdev, dev);
 }
 
 // 63-bit keys -> the same order in 3 b bits: the fields of coordinates |c| <= m (2^b > 2 m).
@@ -733,13 +808,6 @@ __global__ void dedup_emit_kernel(const uint32_t* idx, const int64_t* n, const f
   const uint32_t s = idx[k];
   ou[k] = u[s]; ov[k] = v[s]; ow[k] = w[s];
 }
-
-// Device counters of a table pass, read back in one copy.
-struct DedupCounters {
-  int bad, overflow;  // keys out of range; a key found no slot
-  int maxdev, pad;    // largest |coordinate| among the unique keys
-  int64_t n;          // unique keys
-};
 
 // Sort n unique (key, row) pairs by key, k1/i1 -> k0/i0 (k1 is rewritten with shorter keys).
 static int sort_unique(uint64_t* k1, uint64_t* k0, uint32_t* i1, uint32_t* i0, int64_t n, int maxdev, void* cub_temp,
@@ -953,8 +1021,8 @@ int viss_dedup_uvw(float* u, float* v, float* w, int64_t K, int64_t* count_out, 
     VISS_LAUNCH_CHECK("dedup_table_init_kernel");
     dedup_hash_kernel<<<nb, 256, 0, st>>>(u, v, w, K, p.k0, p.i0, (uint64_t)(T - 1), &p.cnt->bad, &p.cnt->overflow);
     VISS_LAUNCH_CHECK("dedup_hash_kernel");
-    unique_compact_kernel<<<(unsigned)((T + COMPACT_SLOTS - 1) / COMPACT_SLOTS), 256, 0, st>>>(
-        p.k0, p.i0, T, p.k1, p.i1, (unsigned long long*)&p.cnt->n, &p.cnt->maxdev);
+    unique_compact_kernel<<<(unsigned)((T + COMPACT_SLOTS - 1) / COMPACT_SLOTS), 256, 0, st>>>(p.k0, p.i0, T, p.k1, p.i1,
+                                                                                            p.cnt);
     VISS_LAUNCH_CHECK("unique_compact_kernel");
     DedupCounters h{};
     VISS_CUDA(cudaMemcpyAsync(&h, p.cnt, sizeof(h), cudaMemcpyDeviceToHost, st));
@@ -1034,30 +1102,41 @@ int viss_unique_uvw(const float* pos, int64_t S, int32_t nsat, int ordered, doub
   int run = UNIQUE_RUN;
   while (run > UNIQUE_RUN_MIN && S / run * nup < (int64_t)device_sm_count() * UNIQUE_CTAS * 256 * 4) run >>= 1;
   const int64_t threads = (S + run - 1) / run * nup;
-  // First a table for about one unique row in eight, between 2^22 slots (50 MB: it stays in
-  // L2, 403,200 snapshots: initialising, inserting and compacting 941 -> 226 us against 2^25
-  // slots) and 2^25 (an orbit campaign's few tens of millions of unique rows), larger
-  // ones while it fills, up to the workspace's.
-  int64_t T = (int64_t)1 << 22;
-  while (T < ((int64_t)1 << 25) && T < K / 8) T <<= 1;
-  if (T > p.T) T = p.T;
+  // First a table that the rows expected of a sample fill to a half at most: 2^22 slots (50 MB, which stay
+  // in L2) to 2^25 (an orbit campaign's few tens of millions of unique rows); then larger ones while
+  // it fills, up to the workspace's.  A size from the number of rows alone is too large for 403,200
+  // snapshots at 10 MHz (2^25 slots: initialising, inserting and compacting 941 us, 226 with 2^22) or too
+  // small at 30 MHz (2^22 slots 0.93 full: the pass was repeated, 3,170 us against 890), and far too
+  // small for positions that share no row (100,003 snapshots: 10.2 against 1.8 ms).  The sample takes 5 us and
+  // its launch; the size stays on the device.
+  const int64_t first = p.T < ((int64_t)1 << 25) ? p.T : (int64_t)1 << 25;
+  int64_t lo = (int64_t)1 << 22 < first ? (int64_t)1 << 22 : first, hi = first;
+  const int64_t steps = sampled_steps(S);
+  const int resident = device_sm_count() * 8;
   DedupCounters h{};
-  for (;; T = T << 3 < p.T ? T << 3 : p.T) {
+  for (;;) {
     VISS_CUDA(cudaMemsetAsync(p.cnt, 0, sizeof(DedupCounters), st));
-    dedup_table_init_kernel<<<(unsigned)((T + 255) / 256), 256, 0, st>>>(p.tkeys, p.tidx, T);
-    VISS_LAUNCH_CHECK("dedup_table_init_kernel");
-    unique_insert_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(
-        pos, S, nsat, ordered, run, lambda_m, scale, p.tkeys, p.tidx, (uint64_t)(T - 1), &p.cnt->bad, &p.cnt->overflow);
+    if (lo < hi) {
+      const int64_t samples = (S + SAMPLE_STRIDE - 1) / SAMPLE_STRIDE * nup;
+      unique_sample_kernel<<<(unsigned)((samples + 255) / 256), 256, 0, st>>>(pos, S, nsat, ordered, lambda_m, scale, p.cnt);
+      VISS_LAUNCH_CHECK("unique_sample_kernel");
+    }
+    unique_table_kernel<<<(unsigned)resident, 256, 0, st>>>(p.tkeys, p.tidx, S, npairs, steps, (uint32_t)lo, (uint32_t)hi, p.cnt);
+    VISS_LAUNCH_CHECK("unique_table_kernel");
+    unique_insert_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(pos, S, nsat, ordered, run, lambda_m, scale,
+                                                                           p.tkeys, p.tidx, p.cnt);
     VISS_LAUNCH_CHECK("unique_insert_kernel");
-    unique_compact_kernel<<<(unsigned)((T + COMPACT_SLOTS - 1) / COMPACT_SLOTS), 256, 0, st>>>(
-        p.tkeys, p.tidx, T, p.k1, p.i1, (unsigned long long*)&p.cnt->n, &p.cnt->maxdev);
+    const int64_t tiles = (hi + COMPACT_SLOTS - 1) / COMPACT_SLOTS;
+    unique_compact_kernel<<<(unsigned)(tiles < resident ? tiles : resident), 256, 0, st>>>(p.tkeys, p.tidx, 0, p.k1, p.i1,
+                                                                                        p.cnt);
     VISS_LAUNCH_CHECK("unique_compact_kernel");
     VISS_CUDA(cudaMemcpyAsync(&h, p.cnt, sizeof(h), cudaMemcpyDeviceToHost, st));
     VISS_CUDA(cudaStreamSynchronize(st));
     if (h.bad) return fail(VISS_ERR_RANGE, "uvw beyond |x| < 2^20 cannot be keyed");
     if (!h.overflow) break;
-    if (T == p.T)
+    if (h.slots == p.T)
       return fail(VISS_ERR_RANGE, "more unique uvw than the table holds: use viss_baseline_uvw + viss_dedup_uvw");
+    lo = hi = (int64_t)h.slots << 3 < p.T ? (int64_t)h.slots << 3 : p.T;
   }
   const int64_t n = h.n;
   *count_out = n;
