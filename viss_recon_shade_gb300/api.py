@@ -365,21 +365,32 @@ def tuning_candidates() -> list:
     return out
 
 
+def _distinct(cfg: DftConfig, t: Tuning) -> Tuning:
+    """The form of a tuning that a pass of cfg takes: the geometric reconstruction has no row
+    tiles (bits 1 to 3 of tile), only the vis kernel's sky tile (bit 0) matters."""
+    return replace(t, tile=t.tile & 1) if cfg.recon_mask == RECON_MASK_GEOMETRIC else t
+
+
 _TUNED: dict = {}
 
 
 def autotune(batch: ChannelBatch, candidates=None, reps: int = 1, use_cache: bool = True) -> Tuning:
     """Time vis + recon of ``batch`` under each candidate Tuning (CUDA events on the current
-    stream, after one warm-up run each) and keep the fastest on the batch.  Results are cached
-    per device and batch shape (channel row counts, J, mask and precision)."""
+    stream, after one warm-up run each) and keep the fastest on the batch.  Candidates that are the
+    same pass for this batch's masks are timed once and share the time.  Results are cached per
+    device and batch shape (channel row counts, J, mask and precision)."""
     key = (torch.cuda.get_device_name(batch.u.device), tuple(batch.row_off.tolist()), batch.J, batch.cfg.mask,
            batch.cfg.recon_mask, batch.cfg.precision)
     if use_cache and key in _TUNED:
         batch.set_tuning(_TUNED[key][0])
         return _TUNED[key][0]
     cands = list(candidates) if candidates is not None else tuning_candidates()
-    times = []
+    times, timed = [], {}
     for t in cands:
+        form = _distinct(batch.cfg, t)
+        if form in timed:
+            times.append(timed[form])
+            continue
         batch.set_tuning(t)
         batch.step()
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -388,7 +399,8 @@ def autotune(batch: ChannelBatch, candidates=None, reps: int = 1, use_cache: boo
             batch.step()
         e1.record()
         e1.synchronize()
-        times.append(e0.elapsed_time(e1) / reps)
+        timed[form] = e0.elapsed_time(e1) / reps
+        times.append(timed[form])
     best = cands[min(range(len(cands)), key=times.__getitem__)]
     _TUNED[key] = (best, list(zip(cands, times)))
     batch.set_tuning(best)
