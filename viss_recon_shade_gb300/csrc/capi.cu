@@ -249,14 +249,6 @@ static void plan_segments(RecPlan& p, const viss_dft_cfg& cfg, const Batch& bt, 
   // different parts of the orbit (10 MHz recon: 4 items 191 ms, 8 176 ms, 32 167 ms, 64 165 ms)
   const int64_t target = (tn.rec_items > 0 ? tn.rec_items : 64) * planned_ctas(tn, rec_ctas(cfg.recon_mask, p.comp));
   int64_t L = p.npb > 0 ? (p.K * p.npb + target - 1) / target : p.K;
-  // A small pass has fewer than 4 segments of REC_Q rows per CTA: shorter ones, down to
-  // REC_MIN_ROWS, so that every SM has work.  3,360 rows x 2,048 pixels: 58 -> 20 us;
-  // 28,672 x 12,288: REF windows 256 rows 190 us, 128 rows 184 us.
-  if (tn.rec_items <= 0 && L < unit) {
-    while (unit > REC_MIN_ROWS && p.K * p.npb < 4 * (target / 64) * unit) unit >>= 1;
-    L = unit;
-  }
-  L = round_up(L > unit ? L : unit, unit);
   auto count = [&](int64_t len) {
     int64_t n = 0;
     for (int c = 0; c < nch; ++c) {
@@ -265,7 +257,36 @@ static void plan_segments(RecPlan& p, const viss_dft_cfg& cfg, const Batch& bt, 
     }
     return n;
   };
-  while (count(L) > VISS_MAX_SEG) L = round_up(L + (L > 256 ? L / 4 : 0) + 1, unit);
+  auto bounded = [&](int64_t len, int64_t step) {  // at most VISS_MAX_SEG segments
+    len = round_up(len > step ? len : step, step);
+    while (count(len) > VISS_MAX_SEG) len = round_up(len + (len > 256 ? len / 4 : 0) + 1, step);
+    return len;
+  };
+  // A small pass has fewer than 4 segments of REC_Q rows per CTA: shorter ones, down to
+  // REC_MIN_ROWS, so that every SM has work.  3,360 rows x 2,048 pixels: 58 -> 20 us;
+  // 28,672 x 12,288: REF windows 256 rows 190 us, 128 rows 184 us.
+  const int64_t ctas = planned_ctas(tn, rec_ctas(cfg.recon_mask, p.comp));
+  if (tn.rec_items <= 0 && L < unit) {
+    while (unit > REC_MIN_ROWS && p.K * p.npb < 4 * ctas * unit) unit >>= 1;
+    // Many channels of few rows each fill the chip whole, or nearly; cut, each has partial sums to be
+    // written, read and added.  A CTA's row of 1,024 pixels takes ~64 ns; in these rows a
+    // pass takes its items per SM x their rows, the reduction ~60 and one per 8,000 partial sums
+    // (fitted to passes of 1 to 64 channels of 20 to 30,000 rows x 1,024 to 40,000 pixels: within 2 % of
+    // the best length on average, 24 % at most).  64 channels x 100 rows x 20,164 pixels: cut 148 us,
+    // whole 84; 16 x 100 x 20,164 55 and 41.  The geometric kernel's items are warps: cut is better
+    // there throughout.
+    int64_t used = 0;
+    for (int c = 0; c < nch; ++c) used += bt.ch.row_off[c + 1] > bt.ch.row_off[c];
+    auto cost = [&](int64_t len, int64_t step) {
+      const int64_t n = count(bounded(len, step)), items = n * p.npb;
+      const double sms = (double)device_sm_count(), rows = (double)p.K / (double)n;
+      const double each = (items <= ctas ? std::ceil(items / sms) : items / sms) * rows;
+      return n > used ? each + 60.0 + (double)n * (double)p.J / 8000.0 : each;
+    };
+    if (!p.geo && unit < REC_Q && p.K > 0 && count(REC_Q) <= 2 * used && cost(REC_Q, REC_Q) <= cost(unit, unit)) unit = REC_Q;
+    L = unit;
+  }
+  L = bounded(L, unit);
   // With four items per CTA or more, segment i of a channel's n holds rows up to
   // 1.8 x - 0.8 x^2 of them (x = i / n): from 1.8 of the mean down to 0.2.  Taken longest first,
   // the short ones level the last wave, which equal ones leave up to half empty (the number
@@ -274,7 +295,6 @@ static void plan_segments(RecPlan& p, const viss_dft_cfg& cfg, const Batch& bt, 
   // 1,835,008 x 196,608 150.0 -> 148.4 ms; REF windows 28,672 x 12,321 187.7 -> 183.1 us; 1.9 x - 0.9 x^2
   // is the same within 0.3 %.  Fewer items than that all start at once, and the longest decides:
   // 3,360 x 2,048 17.6 -> 23.1 us, so there they stay equal.
-  const int64_t ctas = planned_ctas(tn, rec_ctas(cfg.recon_mask, p.comp));
   const int64_t g = count(L) * p.npb >= 4 * ctas ? 8 : 0;
   auto bound = [g](int64_t kc, int64_t i, int64_t n) { return kc * ((10 + g) * i * n - g * i * i) / (10 * n * n); };
   struct Seg { int64_t lo, hi; int ch, idx; };
