@@ -269,19 +269,20 @@ static void plan_segments(RecPlan& p, const viss_dft_cfg& cfg, const Batch& bt, 
   if (tn.rec_items <= 0 && L < unit) {
     while (unit > REC_MIN_ROWS && p.K * p.npb < 4 * ctas * unit) unit >>= 1;
     // Many channels of few rows each fill the chip whole, or nearly; cut, each has partial sums to be
-    // written, read and added.  A CTA's row of 1,024 pixels takes ~64 ns; in these rows a
-    // pass takes its items per SM x their rows, the reduction ~60 and one per 8,000 partial sums
-    // (fitted to passes of 1 to 64 channels of 20 to 30,000 rows x 1,024 to 40,000 pixels: within 2 % of
-    // the best length on average, 24 % at most).  64 channels x 100 rows x 20,164 pixels: cut 148 us,
-    // whole 84; 16 x 100 x 20,164 55 and 41.  The geometric kernel's items are warps: cut is better
-    // there throughout.
+    // written, read and added.  In rows of an SM (1,024 pixels of one, ~64 ns; 1.3 with REF
+    // windows) a pass takes the rows of an SM's items, at least 1.5 times an item's for one that has
+    // an SM to itself, and the reduction 100 and one per 12,000 partial sums (fitted to 348 passes of 1 to
+    // 64 channels of 20 to 30,000 rows x 1,024 to 40,000 pixels: within 2 % of the best length on average,
+    // 19 % at most; the pass it was wrong for takes 25 us).  64 channels x 100 rows x 20,164 pixels:
+    // cut 148 us, whole 84; 16 x 100 x 20,164 55 and 41.  The geometric kernel's items are
+    // warps: cut is better there throughout.
     int64_t used = 0;
     for (int c = 0; c < nch; ++c) used += bt.ch.row_off[c + 1] > bt.ch.row_off[c];
     auto cost = [&](int64_t len, int64_t step) {
       const int64_t n = count(bounded(len, step)), items = n * p.npb;
-      const double sms = (double)device_sm_count(), rows = (double)p.K / (double)n;
-      const double each = (items <= ctas ? std::ceil(items / sms) : items / sms) * rows;
-      return n > used ? each + 60.0 + (double)n * (double)p.J / 8000.0 : each;
+      const double each = (double)items / device_sm_count(), per_sm = items <= ctas ? std::ceil(each) : each;
+      const double rows = (per_sm > 1.5 ? per_sm : 1.5) * (double)p.K / (double)n * (p.ref ? 1.3 : 1.0);
+      return n > used ? rows + 100.0 + (double)n * (double)p.J / 12000.0 : rows;
     };
     if (!p.geo && unit < REC_Q && p.K > 0 && count(REC_Q) <= 2 * used && cost(REC_Q, REC_Q) <= cost(unit, unit)) unit = REC_Q;
     L = unit;
