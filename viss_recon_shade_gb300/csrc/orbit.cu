@@ -374,12 +374,28 @@ __device__ __forceinline__ float baseline_coord(float diff, double lambda, float
   return ceil_quotient_exact(diff, lambda);
 }
 
+// 1e3 / lambda as a float pair hi + lo (to 2^-48)
+inline float2 scale_pair(double lambda) {
+  const double s = 1e3 / lambda;
+  const float hi = (float)s;
+  return make_float2(hi, (float)(s - (double)hi));
+}
+
+// One baseline coordinate of a position difference: the FP32 positions' (baseline_coord), or of FP64
+// positions ceil(diff * 1e3 / lambda), and without the ceil diff * (1e3 / lambda): one FP64 product where
+// the quotient's division was ten operations or more (the float result differs where the two FP64 values
+// straddle a rounding boundary, a few in 10^6).
+template <class T>
+__device__ __forceinline__ float baseline_value(T diff, double lambda, double scale64, float2 scale, int rounding) {
+  if (sizeof(T) == sizeof(double))
+    return rounding ? (float)ceil((double)diff * 1e3 / lambda) : (float)((double)diff * scale64);
+  return baseline_coord((float)diff, lambda, scale, rounding);
+}
+
 // Baselines of a block's snapshots: their positions and the (m, n) of every pair are staged in
 // shared memory, then a thread forms every BASE_THREADS-th row.  The rows are written in order
-// (20 B each: the bound once the pair and the division are off the rows' path).  FP64
-// positions without the ceil take (p_n - p_m) * (1e3 / lambda): one FP64 product where
-// the quotient's division was ten or more (the float result differs where the two FP64 values
-// straddle a rounding boundary, a few in 10^6).  65,536 snapshots x 28 pairs: 122 -> 34 us.
+// (20 B each: the bound once the pair and the division are off the rows' path).
+// 65,536 snapshots x 28 pairs: 122 -> 35 us.
 constexpr int BASE_THREADS = 256;
 constexpr int BASE_MAX_PAIRS = 32 * 31;
 
@@ -408,18 +424,77 @@ __global__ void __launch_bounds__(BASE_THREADS) baseline_uvw_kernel(const T* pos
     const T* const pn = s_pos + (ls * nsat + (pq >> 16)) * 3;
     float out[3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const T diff = pn[c] - pm[c];
-      if (sizeof(T) == sizeof(double))
-        out[c] = rounding ? (float)ceil((double)diff * 1e3 / lambda) : (float)((double)diff * scale64);
-      else
-        out[c] = baseline_coord((float)diff, lambda, scale, rounding);
-    }
+    for (int c = 0; c < 3; ++c) out[c] = baseline_value<T>(pn[c] - pm[c], lambda, scale64, scale, rounding);
     const int64_t k = g0 * npairs + i;
     u[k] = out[0]; v[k] = out[1]; w[k] = out[2];
     if (snap) snap[k] = (int32_t)(g0 + ls);
     if (pair) pair[k] = pq;
   }
+}
+
+// A thread per row, nothing staged: for the coordinates that take an FP64 division (FP32 positions
+// without the ceil, FP64 ones with it).  Those are bound by the FP64 pipe whatever is staged, and small
+// passes by the chain of a thread's divisions: 120 snapshots x 56 pairs in blocks of 2,048 staged rows
+// take 23 us, 6 here; 16,800 x 56 78 and 62.
+template <class T>
+__global__ void __launch_bounds__(BASE_THREADS) baseline_rows_kernel(const T* pos, int64_t K, int nsat, int ordered, int npairs,
+                                                                    uint64_t magic, double lambda, float2 scale,
+                                                                    int rounding, float* u, float* v, float* w,
+                                                                    int32_t* snap, int32_t* pair) {
+  const int64_t k = (int64_t)blockIdx.x * BASE_THREADS + threadIdx.x;
+  if (k >= K) return;
+  // k / npairs by a multiply-high (magic = ceil(2^64 / npairs), 0 for one pair), corrected once
+  int64_t g = magic ? (int64_t)__umul64hi((uint64_t)k, magic) : k;
+  int q = (int)(k - g * npairs);
+  if (q < 0) { --g; q += npairs; }
+  if (q >= npairs) { ++g; q -= npairs; }
+  int m, n;
+  pair_of(q, nsat, ordered, &m, &n);
+  float out[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+    out[c] = baseline_value<T>(pos[(g * nsat + n) * 3 + c] - pos[(g * nsat + m) * 3 + c], lambda, 0.0, scale, rounding);
+  u[k] = out[0]; v[k] = out[1]; w[k] = out[2];
+  if (snap) snap[k] = (int32_t)g;
+  if (pair) pair[k] = m | (n << 16);
+}
+
+template <class T>
+static int launch_baselines(const T* pos, int64_t S, int nsat, int ordered, int npairs, double lambda, int rounding, float* u,
+                            float* v, float* w, int32_t* snap, int32_t* pair, cudaStream_t st) {
+  const int64_t K = S * npairs;
+  const float2 scale = scale_pair(lambda);
+  const bool fp64 = sizeof(T) == sizeof(double);
+  if (fp64 == (rounding != 0)) {
+    const int64_t blocks = (K + BASE_THREADS - 1) / BASE_THREADS;
+    if (blocks > (int64_t)INT32_MAX) return fail(VISS_ERR_RANGE, "too many baselines");
+    const uint64_t magic = npairs > 1 ? ~0ull / (uint64_t)npairs + 1 : 0;
+    baseline_rows_kernel<T><<<(unsigned)blocks, BASE_THREADS, 0, st>>>(pos, K, nsat, ordered, npairs, magic, lambda, scale,
+                                                                      rounding, u, v, w, snap, pair);
+    VISS_LAUNCH_CHECK("baseline_rows_kernel");
+    return VISS_OK;
+  }
+  // Rows a block: one a thread where the FP64 products bind (65,536 x 28: 35 us, 37 at 2,048); FP32
+  // up to 2,048 in passes of four blocks an SM and more, where a thread's rows share its staging
+  // (200,000 x 56: 256 rows 112 us, 512 72, 1,024 64, 2,048 55; 1,024 x 56: 5.0, 5.0, 5.1, 6.3).
+  // At most 24 KB of positions.
+  int64_t rows = BASE_THREADS;
+  if (!fp64 && K > 1 << 17) {  // four blocks of BASE_THREADS on 128 SMs: smaller passes take the least
+    rows = K / (4 * (int64_t)device_sm_count());
+    rows = rows < BASE_THREADS ? BASE_THREADS : rows > 2048 ? 2048 : rows;
+  }
+  int per_block = (int)rows / npairs;
+  if (per_block > 1024 / nsat) per_block = 1024 / nsat;
+  if (per_block < 1) per_block = 1;
+  if (per_block > S) per_block = (int)S;
+  const int64_t blocks = (S + per_block - 1) / per_block;
+  if (blocks > (int64_t)INT32_MAX) return fail(VISS_ERR_RANGE, "too many snapshots");
+  FastDiv by_npairs;
+  by_npairs.set(npairs);
+  baseline_uvw_kernel<T><<<(unsigned)blocks, BASE_THREADS, sizeof(T) * per_block * nsat * 3, st>>>(
+      pos, S, nsat, ordered, npairs, per_block, by_npairs, lambda, 1e3 / lambda, scale, rounding, u, v, w, snap, pair);
+  VISS_LAUNCH_CHECK("baseline_uvw_kernel");
+  return VISS_OK;
 }
 
 // ---------------------------------------------------------------- dedup
@@ -850,13 +925,6 @@ struct DedupPlan {
   }
 };
 
-// 1e3 / lambda as a float pair hi + lo (to 2^-48)
-inline float2 scale_pair(double lambda) {
-  const double s = 1e3 / lambda;
-  const float hi = (float)s;
-  return make_float2(hi, (float)(s - (double)hi));
-}
-
 // Workspace of viss_unique_uvw: a table of up to T = 2K slots (pow2, 2^10 ..
 // 2^28), the compacted (key, first row) pairs and the CUB scratch.
 struct UniquePlan {
@@ -966,26 +1034,8 @@ int viss_baseline_uvw(const float* pos, const double* pos64, int64_t S, int32_t 
   const int64_t K = S * npairs;
   if (K == 0) return VISS_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // ~2,048 rows a block (several rows a thread share its staging), and at most 24 KB of positions
-  int per_block = 2048 / npairs;
-  if (per_block > 1024 / nsat) per_block = 1024 / nsat;
-  if (per_block < 1) per_block = 1;
-  if (per_block > S) per_block = (int)S;
-  const int64_t blocks = (S + per_block - 1) / per_block;
-  if (blocks > (int64_t)INT32_MAX) return fail(VISS_ERR_RANGE, "too many snapshots");
-  FastDiv by_npairs;
-  by_npairs.set(npairs);
-  const size_t elems = (size_t)per_block * nsat * 3;
-  if (pos64)
-    baseline_uvw_kernel<double><<<(unsigned)blocks, BASE_THREADS, elems * sizeof(double), st>>>(
-        pos64, S, nsat, ordered, npairs, per_block, by_npairs, lambda_m, 1e3 / lambda_m, scale_pair(lambda_m), rounding,
-        u, v, w, snap, pair);
-  else
-    baseline_uvw_kernel<float><<<(unsigned)blocks, BASE_THREADS, elems * sizeof(float), st>>>(
-        pos, S, nsat, ordered, npairs, per_block, by_npairs, lambda_m, 1e3 / lambda_m, scale_pair(lambda_m), rounding, u,
-        v, w, snap, pair);
-  VISS_LAUNCH_CHECK("baseline_uvw_kernel");
-  return VISS_OK;
+  return pos64 ? launch_baselines(pos64, S, nsat, ordered, npairs, lambda_m, rounding, u, v, w, snap, pair, st)
+               : launch_baselines(pos, S, nsat, ordered, npairs, lambda_m, rounding, u, v, w, snap, pair, st);
 }
 
 size_t viss_dedup_uvw_workspace(int64_t K) {
