@@ -663,15 +663,20 @@ __device__ __forceinline__ void row_keys(const float* d, double lambda, float2 s
 }
 
 // How many rows will be inserted: the rows whose key differs from their snapshot's before, counted over
-// SAMPLE_STEPS of every SAMPLE_STRIDE snapshots.  They bound the unique rows, closely for an orbit, where a
+// SAMPLE_STEPS of every 256 snapshots (fewer where that is over SAMPLE_CHUNKS times).  They bound the unique rows, closely for an orbit, where a
 // key seldom comes back (403,200 snapshots of 8 satellites: 1.27 of them at 1 MHz, 1.02 at 30 MHz).
-constexpr int SAMPLE_STEPS = 4, SAMPLE_STRIDE = 256;
+constexpr int SAMPLE_STEPS = 4, SAMPLE_CHUNKS = 8192;
 
-__global__ void __launch_bounds__(256) unique_sample_kernel(const float* __restrict__ pos, int64_t S, int nsat, int ordered,
-                                                            double lambda, float2 scale, DedupCounters* cnt) {
+static int64_t sample_stride(int64_t S) {
+  const int64_t least = (S + SAMPLE_CHUNKS - 1) / SAMPLE_CHUNKS;
+  return least > 256 ? least : 256;
+}
+
+__global__ void __launch_bounds__(256) unique_sample_kernel(const float* __restrict__ pos, int64_t S, int64_t stride, int nsat,
+                                                            int ordered, double lambda, float2 scale, DedupCounters* cnt) {
   const int nup = nsat * (nsat - 1) / 2;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t chunk = t / nup, g0 = chunk * SAMPLE_STRIDE;
+  const int64_t chunk = t / nup, g0 = chunk * stride;
   int changes = 0;
   if (g0 + 1 < S) {
     int m, n;
@@ -700,7 +705,7 @@ __global__ void __launch_bounds__(256) unique_sample_kernel(const float* __restr
 
 // Sampled steps of one satellite pair.
 static int64_t sampled_steps(int64_t S) {
-  const int64_t whole = (S - 1) / SAMPLE_STRIDE, rest = (S - 1) % SAMPLE_STRIDE;
+  const int64_t whole = (S - 1) / sample_stride(S), rest = (S - 1) % sample_stride(S);
   return whole * SAMPLE_STEPS + (rest < SAMPLE_STEPS ? rest : SAMPLE_STEPS);
 }
 
@@ -1167,8 +1172,9 @@ int viss_unique_uvw(const float* pos, int64_t S, int32_t nsat, int ordered, doub
   for (;;) {
     VISS_CUDA(cudaMemsetAsync(p.cnt, 0, sizeof(DedupCounters), st));
     if (lo < hi) {
-      const int64_t samples = (S + SAMPLE_STRIDE - 1) / SAMPLE_STRIDE * nup;
-      unique_sample_kernel<<<(unsigned)((samples + 255) / 256), 256, 0, st>>>(pos, S, nsat, ordered, lambda_m, scale, p.cnt);
+      const int64_t stride = sample_stride(S), samples = (S + stride - 1) / stride * nup;
+      unique_sample_kernel<<<(unsigned)((samples + 255) / 256), 256, 0, st>>>(pos, S, stride, nsat, ordered, lambda_m, scale,
+                                                                             p.cnt);
       VISS_LAUNCH_CHECK("unique_sample_kernel");
     }
     unique_table_kernel<<<(unsigned)resident, 256, 0, st>>>(p.tkeys, p.tidx, S, npairs, steps, (uint32_t)lo, (uint32_t)hi, p.cnt);
